@@ -223,75 +223,4 @@ cudaError_t launch_adjoint(const Tess &t, int nsteps, int mode, const AdjointPla
 #undef CPAB_ADJ
 }
 
-// ------------------------------ finalize -------------------------------------
-template <int N, int MODE>
-__global__ void __launch_bounds__(256)
-    k_finalize(int nC, Steps st, const float *__restrict__ partials, int parts,
-               const float *__restrict__ A, const float *__restrict__ basis, int d,
-               float *__restrict__ dtheta) {
-    constexpr int P = N * (N + 1);
-    extern __shared__ float4 smem4[];
-    float *g = reinterpret_cast<float *>(smem4);
-    const int th = blockIdx.x, tid = threadIdx.x, B = blockDim.x;
-    const int G = nC * P;
-    const float *src = partials + (long long)th * parts * G;
-    for (int i = tid; i < G; i += B) {
-        // four interleaved sums (loads in flight), combined in a fixed order
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-        int q = 0;
-        for (; q + 4 <= parts; q += 4) {
-            s0 += __ldg(src + (long long)q * G + i);
-            s1 += __ldg(src + (long long)(q + 1) * G + i);
-            s2 += __ldg(src + (long long)(q + 2) * G + i);
-            s3 += __ldg(src + (long long)(q + 3) * G + i);
-        }
-        for (; q < parts; ++q) s0 += __ldg(src + (long long)q * G + i);
-        g[i] = (s0 + s1) + (s2 + s3);
-    }
-    __syncthreads();
-    finish_theta<N, MODE>(g, g + round4(G), A + (long long)th * G, nC, st, basis, d,
-                          dtheta + (long long)th * d);
-}
-
-cudaError_t launch_finalize(const Tess &t, int nsteps, int mode, const float *partials, int parts,
-                            const float *A, const float *basis, int d, int n_theta,
-                            float *dtheta, cudaStream_t s) {
-    if (n_theta == 0) return cudaSuccess;
-    const int P = t.ndim * (t.ndim + 1);
-    const int block = 256;
-    const size_t smem = ((size_t)round4(t.nC * P) + block) * sizeof(float);
-    const Steps st = make_steps(nsteps);
-#define CPAB_FIN(N, M)                                                                         \
-    {                                                                                          \
-        auto kern = k_finalize<N, M>;                                                          \
-        if (smem > 48 * 1024) {                                                                \
-            cudaError_t e = cudaFuncSetAttribute(                                              \
-                kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                 \
-            if (e != cudaSuccess) return e;                                                    \
-        }                                                                                      \
-        kern<<<n_theta, block, smem, s>>>(t.nC, st, partials, parts, A, basis, d, dtheta);     \
-        return cudaGetLastError();                                                             \
-    }
-    if (mode == kFinalizeDirect) {   // the partials are dL/dA (exact-flow adjoint)
-        switch (t.ndim) {
-            case 1: CPAB_FIN(1, 3)
-            case 2: CPAB_FIN(2, 3)
-            default: CPAB_FIN(3, 3)
-        }
-    }
-    if (mode != 1) {   // modes 0 and 2: the midpoint sensitivity's cell map
-        switch (t.ndim) {
-            case 1: CPAB_FIN(1, 0)
-            case 2: CPAB_FIN(2, 0)
-            default: CPAB_FIN(3, 0)
-        }
-    }
-    switch (t.ndim) {
-        case 1: CPAB_FIN(1, 1)
-        case 2: CPAB_FIN(2, 1)
-        default: CPAB_FIN(3, 1)
-    }
-#undef CPAB_FIN
-}
-
 }  // namespace cpab

@@ -570,184 +570,4 @@ __device__ __forceinline__ void adjoint_epilogue(const AdjSmem<N, CT> &sm, int n
     }
 }
 
-// Frechet derivative of expm at Y in direction E, by a truncated Horner
-// recursion on Y/2^s, E/2^s followed by s squarings:
-//   R_{k-1} = I + (Y/k) R_k,  dR_{k-1} = (E/k) R_k + (Y/k) dR_k,
-//   then  L <- L R + R L,  R <- R R.
-// Rout receives R = expm(Y) (the overload without it drops R).
-template <int K>
-__device__ __forceinline__ void frechet_expm(const float (&Y0)[K][K], const float (&E0)[K][K],
-                                             float (&L)[K][K], float (&Rout)[K][K]) {
-    float norm = 0.f;
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-        float s = 0.f;
-#pragma unroll
-        for (int i = 0; i < K; ++i) s += fabsf(Y0[i][j]);
-        norm = fmaxf(norm, s);
-    }
-    int sq = 0;
-    if (norm > 0.5f) sq = min(64, (int)ceilf(log2f(norm / 0.5f)));
-    const float sc = ldexpf(1.f, -sq);
-    float Y[K][K], E[K][K], R[K][K], D[K][K];
-#pragma unroll
-    for (int i = 0; i < K; ++i)
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            Y[i][j] = Y0[i][j] * sc;
-            E[i][j] = E0[i][j] * sc;
-            R[i][j] = (i == j) ? 1.f : 0.f;
-            D[i][j] = 0.f;
-        }
-    for (int k = 12; k >= 1; --k) {
-        const float r = 1.f / (float)k;
-        float nR[K][K], nD[K][K];
-#pragma unroll
-        for (int i = 0; i < K; ++i)
-#pragma unroll
-            for (int j = 0; j < K; ++j) {
-                float a = 0.f, b = 0.f;
-#pragma unroll
-                for (int m = 0; m < K; ++m) {
-                    a = fmaf(Y[i][m], R[m][j], a);
-                    b = fmaf(E[i][m], R[m][j], fmaf(Y[i][m], D[m][j], b));
-                }
-                nR[i][j] = fmaf(a, r, (i == j) ? 1.f : 0.f);
-                nD[i][j] = b * r;
-            }
-#pragma unroll
-        for (int i = 0; i < K; ++i)
-#pragma unroll
-            for (int j = 0; j < K; ++j) { R[i][j] = nR[i][j]; D[i][j] = nD[i][j]; }
-    }
-    for (int s = 0; s < sq; ++s) {
-        float nR[K][K], nD[K][K];
-#pragma unroll
-        for (int i = 0; i < K; ++i)
-#pragma unroll
-            for (int j = 0; j < K; ++j) {
-                float a = 0.f, b = 0.f;
-#pragma unroll
-                for (int m = 0; m < K; ++m) {
-                    a = fmaf(R[i][m], R[m][j], a);
-                    b = fmaf(D[i][m], R[m][j], fmaf(R[i][m], D[m][j], b));
-                }
-                nR[i][j] = a;
-                nD[i][j] = b;
-            }
-#pragma unroll
-        for (int i = 0; i < K; ++i)
-#pragma unroll
-            for (int j = 0; j < K; ++j) { R[i][j] = nR[i][j]; D[i][j] = nD[i][j]; }
-    }
-#pragma unroll
-    for (int i = 0; i < K; ++i)
-#pragma unroll
-        for (int j = 0; j < K; ++j) L[i][j] = D[i][j];
-#pragma unroll
-    for (int i = 0; i < K; ++i)
-#pragma unroll
-        for (int j = 0; j < K; ++j) Rout[i][j] = R[i][j];
-}
-
-template <int K>
-__device__ __forceinline__ void frechet_expm(const float (&Y0)[K][K], const float (&E0)[K][K],
-                                             float (&L)[K][K]) {
-    float R[K][K];
-    frechet_expm<K>(Y0, E0, L, R);
-}
-
-// Per-theta tail of the finalize kernels, run by one block after the summed
-// cell statistics are in g (shared memory, nC * N*(N+1) floats; red is
-// blockDim.x floats of shared scratch): map them to
-// dL/dA (mode 0: G = h S (I + h/2 [A;0])^T + h^2/2 A_lin^T S; mode 1: adjoint
-// Frechet derivative of expm; mode 3, the exact-flow adjoint: already dL/dA)
-// and contract with the basis, dtheta[k] = sum_i B[i, k] dA[i].
-template <int N, int MODE>
-__device__ __forceinline__ void finish_theta(float *g, float *red, const float *__restrict__ A_th,
-                                             int nC, const Steps &st,
-                                             const float *__restrict__ basis, int d,
-                                             float *__restrict__ dth) {
-    constexpr int P = N * (N + 1);
-    const int tid = threadIdx.x, B = blockDim.x, G = nC * P;
-    if constexpr (MODE == 3) {
-        // the exact-flow adjoint's partials are dL/dA already
-    } else if constexpr (MODE != 1) {
-        // S_c = sum_n lambda_{n+1} [p_n;1]^T  ->
-        // G_c = h S_c (I + h/2 [A_c;0])^T + h^2/2 A_lin^T S_c
-        for (int c = tid; c < nC; c += B) {
-            const float *a = A_th + (long long)c * P;
-            float S[N][N + 1], Gc[N][N + 1];
-#pragma unroll
-            for (int i = 0; i < N; ++i)
-#pragma unroll
-                for (int j = 0; j <= N; ++j) S[i][j] = g[c * P + i * (N + 1) + j];
-#pragma unroll
-            for (int i = 0; i < N; ++i)
-#pragma unroll
-                for (int j = 0; j <= N; ++j) {
-                    float x = 0.f, y = 0.f;
-                    if (j < N) {
-#pragma unroll
-                        for (int k = 0; k <= N; ++k) x = fmaf(S[i][k], a[j * (N + 1) + k], x);
-                    }
-#pragma unroll
-                    for (int r = 0; r < N; ++r) y = fmaf(a[r * (N + 1) + i], S[r][j], y);
-                    Gc[i][j] = fmaf(st.h, fmaf(st.hh, x, S[i][j]), st.hh2 * y);
-                }
-#pragma unroll
-            for (int i = 0; i < N; ++i)
-#pragma unroll
-                for (int j = 0; j <= N; ++j) g[c * P + i * (N + 1) + j] = Gc[i][j];
-        }
-        __syncthreads();
-    } else {
-        const float dt = st.h;
-        // dL/dT_c (top N rows) -> dL/dA_c = dt * [L_exp(X^T, [dL/dT_c; 0])]_{top rows}
-        for (int c = tid; c < nC; c += B) {
-            const float *a = A_th + (long long)c * P;
-            float Y[N + 1][N + 1], E[N + 1][N + 1], L[N + 1][N + 1];
-#pragma unroll
-            for (int i = 0; i <= N; ++i)
-#pragma unroll
-                for (int j = 0; j <= N; ++j) {
-                    Y[j][i] = (i < N) ? dt * a[i * (N + 1) + j] : 0.f;   // Y = X^T
-                    E[i][j] = (i < N) ? g[c * P + i * (N + 1) + j] : 0.f;
-                }
-            frechet_expm<N + 1>(Y, E, L);
-#pragma unroll
-            for (int i = 0; i < N; ++i)
-#pragma unroll
-                for (int j = 0; j <= N; ++j) g[c * P + i * (N + 1) + j] = dt * L[i][j];
-        }
-        __syncthreads();
-    }
-    if (d <= 0) return;
-    if (d > B) {
-        for (int k = tid; k < d; k += B) {
-            float acc = 0.f;
-            for (int i = 0; i < G; ++i) acc = fmaf(__ldg(basis + (long long)i * d + k), g[i], acc);
-            dth[k] = acc;
-        }
-        return;
-    }
-    // d <= B: `groups` threads per basis column each take every groups-th row;
-    // their partial sums are added in group order (red: B floats of shared
-    // memory)
-    const int groups = B / d;
-    const int k = tid % d, gi = tid / d;
-    if (gi < groups) {
-        float acc = 0.f;
-        for (int i = gi; i < G; i += groups)
-            acc = fmaf(__ldg(basis + (long long)i * d + k), g[i], acc);
-        red[tid] = acc;
-    }
-    __syncthreads();
-    if (tid < d) {
-        float acc = 0.f;
-        for (int q = 0; q < groups; ++q) acc += red[q * d + tid];
-        dth[tid] = acc;
-    }
-}
-
 }  // namespace cpab

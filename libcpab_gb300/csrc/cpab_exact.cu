@@ -25,6 +25,7 @@
 //     raises kErrIterLimit and returns its position at that point.
 #include "cpab_adjoint.cuh"
 #include "cpab_expm.cuh"
+#include "cpab_frechet.cuh"
 
 namespace cpab {
 

@@ -92,6 +92,13 @@ constexpr int kFinalizeDirect = 3;
 cudaError_t launch_finalize(const Tess &t, int nsteps, int mode, const float *partials, int parts,
                             const float *A, const float *basis, int d, int n_theta,
                             float *dtheta, cudaStream_t s);
+// The same for ragged sets, whose partials are the slots w + s of the `warps`
+// warps of the adjoint launch (cpab_ragged.cuh); sse_partials / sse (may be
+// null): per-series squared error of the fused 1D MSE; dtheta may be null.
+cudaError_t launch_ragged_finalize(const Tess &t, int nsteps, int mode, const float *partials,
+                                   const int *tile_off, int S, int warps, const float *A,
+                                   const float *basis, int d, float *dtheta,
+                                   const float *sse_partials, float *sse, cudaStream_t s);
 
 // Linear / bilinear / trilinear sampling (libcpab/pytorch/interpolation.py).
 // err: device error word (a timed-out grid-tile copy of the 3D kernel).

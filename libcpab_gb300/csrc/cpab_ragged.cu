@@ -24,7 +24,7 @@
 //     them to partial slot (warp + series).  Warps own contiguous tile ranges,
 //     so series s is touched exactly by warps tile_off[s]/K ..
 //     (tile_off[s+1]-1)/K and the slots of all touched (warp, series) pairs
-//     are distinct.  k_ragged_finalize sums a series' slots in warp order:
+//     are distinct.  k_finalize sums a series' slots in warp order:
 //     deterministic, no atomics.
 //
 // The trajectory arithmetic is that of the other kernels: compensated update
@@ -461,15 +461,8 @@ static cudaError_t launch_ra_ls(const Tess &t, int nsteps, int block, int ppt, i
     const Steps st = make_steps(nsteps);
     kern<<<grid, block, smem, s>>>(t, nsteps, st, S, off, tile_off, ppt, a, ties, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    auto fin = k_ragged_finalize<1, MODE>;
-    const size_t fsmem = ((size_t)round4(t.nC * 2) + 256) * sizeof(float);
-    if (fsmem > 48 * 1024) {
-        e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
-        if (e != cudaSuccess) return e;
-    }
-    fin<<<S, 256, fsmem, s>>>(t.nC, st, S, tile_off, grid * (block / 32), a.partials,
-                              a.sse_partials, a.A, basis, d, dtheta, sse);
-    return cudaGetLastError();
+    return launch_ragged_finalize(t, nsteps, MODE, a.partials, tile_off, S, grid * (block / 32),
+                                  a.A, basis, d, dtheta, a.sse_partials, sse, s);
 }
 
 template <int MODE, typename CT, bool FUSED>

@@ -34,38 +34,4 @@ __device__ __forceinline__ int find_series(const int *tile_off, int S, int t) {
 cudaError_t launch_ragged_plan(int S, const long long *off, long long total, int tpw,
                                int *tile_off, unsigned *err, cudaStream_t s);
 
-// ------------------------------- finalize ------------------------------------
-// One block per series / point set: sum its partial slots in warp order, then
-// the per-theta tail shared with k_finalize (sse: per-series squared error of
-// the fused 1D MSE, may be NULL).
-template <int N, int MODE>
-__global__ void __launch_bounds__(256)
-    k_ragged_finalize(int nC, Steps st, int S, const int *__restrict__ tile_off, int TW,
-                      const float *__restrict__ partials, const float *__restrict__ sse_partials,
-                      const float *__restrict__ A, const float *__restrict__ basis, int d,
-                      float *__restrict__ dtheta, float *__restrict__ sse) {
-    extern __shared__ float4 smem4[];
-    float *g = reinterpret_cast<float *>(smem4);
-    const int s = blockIdx.x, tid = threadIdx.x, B = blockDim.x;
-    const int G = nC * N * (N + 1);
-    const int TT = __ldg(tile_off + S);
-    const int K = max(1, (TT + TW - 1) / TW);
-    const int a = __ldg(tile_off + s), b = __ldg(tile_off + s + 1);
-    const int w0 = a / K, w1 = (b > a) ? (b - 1) / K : w0 - 1;
-    for (int i = tid; i < G; i += B) {
-        float acc = 0.f;
-        for (int w = w0; w <= w1; ++w) acc += __ldg(partials + ((long long)w + s) * G + i);
-        g[i] = acc;
-    }
-    if (sse && tid == 0) {
-        float acc = 0.f;
-        for (int w = w0; w <= w1; ++w) acc += __ldg(sse_partials + (long long)w + s);
-        sse[s] = acc;
-    }
-    __syncthreads();
-    if (dtheta)
-        finish_theta<N, MODE>(g, g + round4(G), A + (long long)s * G, nC, st, basis, d,
-                              dtheta + (long long)s * d);
-}
-
 }  // namespace cpab

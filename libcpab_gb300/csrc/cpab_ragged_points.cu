@@ -296,15 +296,8 @@ static cudaError_t launch_rpa_t(const Tess &t, int nsteps, int S, const long lon
                                    ties, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (d == 0 || !dtheta) return cudaSuccess;
-    auto fin = k_ragged_finalize<N, MODE>;
-    const size_t fsmem = ((size_t)round4(t.nC * N * (N + 1)) + 256) * sizeof(float);
-    if (fsmem > 48 * 1024) {
-        e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
-        if (e != cudaSuccess) return e;
-    }
-    fin<<<S, 256, fsmem, s>>>(t.nC, st, S, tile_off, grid * W, partials, nullptr, A, basis, d,
-                              dtheta, nullptr);
-    return cudaGetLastError();
+    return launch_ragged_finalize(t, nsteps, MODE, partials, tile_off, S, grid * W, A, basis, d,
+                                  dtheta, nullptr, nullptr, s);
 }
 
 cudaError_t launch_ragged_points_backward(const Tess &t, int nsteps, int mode, int S,
