@@ -57,8 +57,9 @@
 namespace cpab {
 
 template <int N, int MODE, typename CT, bool GWG>
-__global__ void __launch_bounds__(256)
-    k_adjoint(Tess t, int nsteps, Steps st, const float *__restrict__ points, int broadcast,
+__global__ void __launch_bounds__(256, step_blocks<N>())
+    k_adjoint(const __grid_constant__ Tess t,
+              int nsteps, Steps st, const float *__restrict__ points, int broadcast,
               long long nP, const float *__restrict__ table, int parts, int tiles,
               const float *__restrict__ gout, float *__restrict__ dpoints,
               float *__restrict__ partials, float *gw_ext, unsigned long long *ties,

@@ -59,6 +59,14 @@ struct Tess {
     int tier2;        // 2D second-tier tie decisions apply (square cells, see cell_2d_tier2)
     int pow2;         // every nc[j] (j < ndim, ndim >= 2) is a power of two: p / inc == p * nc
     float ncf[3];     // nc as float
+    // 2D first tier (cell_2d_quick): w = clamp01(p) qa + qb is the sub-cell
+    // coordinate p nc - 1/2 moved inwards by at most qedge at the domain edges
+    float qa[2], qb;
+    float qhalf;      // largest |w - rint(w)| that decides a square (-1: none does)
+    float qmargin;    // relative margin of its triangle tests
+    // nc * inc (exact in double) and (nc_y - nc_x) * inc_x as float pairs, for
+    // the second tier
+    float nih[2], nil[2], dih, dil;
 };
 
 // The lookup functions are host+device so that a host harness can check the
@@ -99,6 +107,28 @@ inline int tess_init(int ndim, const int *nc, Tess *t) {
     t->tier2 = ndim == 2 && t->inc[0] == t->inc[1];
     for (int j = 0; j < 2; ++j)
         t->tier2 &= (double)nextafterf(t->wlim[j], 0.f) <= (double)t->wlim[j] - 0.000000001;
+    if (ndim == 2) {
+        // see cell_2d_quick for the bounds behind these margins
+        const float nmax = fmaxf(t->ncf[0], t->ncf[1]);
+        const double edge = (double)nmax * nmax * 4.76837158203125e-07;   // nmax^2 2^-21
+        t->qb = (float)(-0.5 + edge);
+        t->qhalf = (float)(0.5 - edge * (1.0 - 1.0 / ((double)nmax + 1.0)));
+        t->qmargin = (nmax + 1.f) * 9.5367431640625e-07f;                 // (nmax + 1) 2^-20
+        bool quick = edge < 0.125;
+        for (int j = 0; j < 2; ++j) {
+            t->qa[j] = (float)((double)t->ncf[j] - 2.0 * edge);
+            const double v = (double)nc[j] * (double)t->inc[j];
+            t->nih[j] = (float)v;
+            t->nil[j] = (float)(v - (double)t->nih[j]);
+            // floats in [nc*inc, wlim) would take the reference's fmod
+            // remainder past the last cell
+            quick &= (double)nextafterf(t->wlim[j], 0.f) < v;
+        }
+        if (!quick) t->qhalf = -1.f;
+        const double dv = (double)(nc[1] - nc[0]) * (double)t->inc[0];
+        t->dih = (float)dv;
+        t->dil = (float)(dv - (double)t->dih);
+    }
     t->pow2 = ndim >= 2;
     for (int j = 0; j < ndim; ++j) t->pow2 &= (t->nc[j] & (t->nc[j] - 1)) == 0;
     if (ndim == 3) {
@@ -138,6 +168,70 @@ CPAB_HD inline int small_float_to_int(float x) {
     return float_bits(CPAB_ADD_RN(x, kRoundMagic)) - kRoundMagicBits;
 }
 
+// Two floats operated on by one instruction (each half is the same IEEE
+// operation as the scalar one).  A packed operation takes the FP32 pipe for
+// two cycles but one issue slot, which is what the issue-bound step loops are
+// short of.
+struct F2 {
+    float x, y;
+};
+#if defined(__CUDA_ARCH__)
+#define CPAB_F2_OP2(name, op)                                                                     \
+    __device__ __forceinline__ F2 name(F2 a, F2 b) {                                              \
+        F2 d;                                                                                     \
+        asm("{\n .reg .b64 a, b, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n " op          \
+            " d, a, b;\n mov.b64 {%0, %1}, d;\n}"                                                 \
+            : "=f"(d.x), "=f"(d.y)                                                                \
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                            \
+        return d;                                                                                 \
+    }
+CPAB_F2_OP2(f2_add, "add.rn.f32x2")
+CPAB_F2_OP2(f2_mul, "mul.rn.f32x2")
+CPAB_F2_OP2(f2_add_rd, "add.rm.f32x2")
+#undef CPAB_F2_OP2
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 d;
+    asm("{\n .reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n"
+        " mov.b64 c, {%6, %7};\n fma.rn.f32x2 d, a, b, c;\n mov.b64 {%0, %1}, d;\n}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+#else
+inline F2 f2_add(F2 a, F2 b) { return {a.x + b.x, a.y + b.y}; }
+inline F2 f2_mul(F2 a, F2 b) { return {a.x * b.x, a.y * b.y}; }
+inline F2 f2_fma(F2 a, F2 b, F2 c) { return {fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
+#endif
+CPAB_HD inline F2 f2_rep(float v) { return {v, v}; }
+// a - b (b negated inside an FMA: exact)
+CPAB_HD inline F2 f2_sub(F2 a, F2 b) { return f2_fma(b, f2_rep(-1.f), a); }
+
+// kRoundMagic + floor(x) for |x| < 2^22 (one add rounded towards -infinity;
+// the sum's ulp is 1)
+CPAB_HD inline float floor_magic(float x) {
+#if defined(__CUDA_ARCH__)
+    return __fadd_rd(x, kRoundMagic);
+#else
+    return (float)(floor((double)x) + (double)kRoundMagic);
+#endif
+}
+CPAB_HD inline F2 f2_floor_magic(F2 x) {
+#if defined(__CUDA_ARCH__)
+    return f2_add_rd(x, f2_rep(kRoundMagic));
+#else
+    return {floor_magic(x.x), floor_magic(x.y)};
+#endif
+}
+
+// clamp to [0, 1], NaN to 0
+CPAB_HD inline float clamp01(float x) {
+#if defined(__CUDA_ARCH__)
+    return __saturatef(x);
+#else
+    return x > 0.f ? (x < 1.f ? x : 1.f) : 0.f;
+#endif
+}
+
 // Division of 32-bit unsigned numerators by a fixed divisor d >= 1 with one
 // multiply-high (Granlund & Montgomery, "Division by invariant integers using
 // multiplication", PLDI 1994): m = floor(2^32 (2^l - d) / d) + 1 with
@@ -173,12 +267,14 @@ CPAB_HD inline unsigned fast_div(unsigned n, const FastDiv &f) {
 // floor(p * nc) with the float product, clamped to [0, nc-1]
 // (cpab_ops.cu:14-19).  Non-finite and huge products saturate like CUDA's
 // float->int conversion: +inf and large values give nc-1, -inf and NaN give 0.
+// One add rounded towards -infinity leaves kRoundMagic + floor(q) (its ulp is
+// 1 for |q| < 2^22); the clamp to [0, nc - 1] on that sum also takes
+// everything beyond (the order is kept) and NaN (to 0).
 CPAB_HD inline int cell_1d(float p, const Tess &t) {
     const float q = CPAB_MUL_RN(p, t.ncf[0]);
-    const float k = round_small(q);
-    float f = (k > q) ? k - 1.f : k;                    // floor, exact for |q| < 2^22
-    f = fminf(fmaxf(f, 0.f), t.ncf[0] - 1.f);          // NaN -> 0
-    return small_float_to_int(f);
+    const float k = floor_magic(q);
+    return float_bits(fminf(fmaxf(k, kRoundMagic), kRoundMagic + (t.ncf[0] - 1.f))) -
+           kRoundMagicBits;
 }
 
 // ------------------------------- 2D ---------------------------------------
@@ -227,9 +323,6 @@ CPAB_HD inline void split_exact(float p, float inc, float rinc, float &fi, float
 // |p * rinc| below this keeps every integer in split_exact exact.
 constexpr float kSplitLimit = 2097152.0f;   // 2^21
 
-// cell_2d_fast's code for "a triangle decision is within its margin".
-constexpr int kTie2 = -2;
-
 // Margin of the FP32 sub-cell tests.  A sub-cell coordinate rem*rinc differs
 // from the reference's double rem/inc by at most 2^-22; a two-term test then
 // carries an error below (1+|x|+|y|) 2^-21 and a three-term test below
@@ -237,9 +330,9 @@ constexpr int kTie2 = -2;
 constexpr float kMargin2 = 1.9073486328125e-06f;   // 2^-19
 constexpr float kMargin3 = 3.814697265625e-06f;    // 2^-18
 
-// FP32 2D lookup with the reference's semantics for every finite point;
-// returns kTie2 when a triangle decision is within its error margin (the
-// second tier may decide it) and -1 in the other deferred cases.
+// FP32 2D lookup with the reference's semantics for every finite point (exact
+// squares, triangle decisions with a margin; the second tier of oblong cells);
+// returns -1 where the FP64 replica must decide.
 //
 // Outside the domain the reference applies its left/right/above/below rules
 // (cpab_ops.cpp:57-90).  Each of them is the in-square triangle test applied
@@ -267,113 +360,178 @@ CPAB_HD inline int cell_2d_fast(float px, float py, const Tess &t) {
     const float y = fmaf(rj, t.rinc[1], fj - cj);
     const float dxy = x - y, sxy = (x + y) - 1.f;
     const float m = kMargin2 * ((1.f + fabsf(x)) + fabsf(y));
-    if (!(fabsf(dxy) > m) || !(fabsf(sxy) > m)) return kTie2;
+    if (!(fabsf(dxy) > m) || !(fabsf(sxy) > m)) return -1;
     // triangle: 0 (dxy >= 0, sxy <= 0), 1 (dxy >= 0, sxy > 0), 2 (dxy < 0,
     // sxy > 0), 3 (dxy < 0, sxy <= 0) = (sxy > 0) xor (dxy < 0 ? 3 : 0)
     const int tri = (sxy > 0.f ? 1 : 0) ^ (dxy < 0.f ? 3 : 0);
     return small_float_to_int(4.f * fmaf(cj, t.ncf[0], ci)) + tri;
 }
 
-// Second tier for triangle decisions inside the FP32 margin, for square
-// cells (inc_x == inc_y, Tess::tier2).  Trajectories that sit on a tie for
-// many steps (zero-boundary domain corners are fixed points up to ~1e-17
-// drift) would otherwise take the FP64 replica at every step.  It follows the
-// reference's branch order (cpab_ops.cpp:57-98) and decides each comparison
-// exactly where that is provable, else returns -1 (FP64 replica):
+// First tier of the 2D lookup: the cell wherever every decision is clear of
+// its margin, else -1.  About half the instructions of cell_2d_fast, because
+// nothing has to be exact: the margins cover the rounding of the products.
+//
+// Square: w = clamp01(p) qa + qb.  Without the inward shift it is p nc - 1/2,
+// whose nearest integer is the square (clamped to the domain by the clamp).
+// The shift moves w by e (1 - 2 p), e = nmax^2 2^-21: at the edges w stays e
+// inside the first or last square, so points on and beyond the domain edge
+// (where zero-boundary trajectories live) are decided, and at an interior line
+// it is off by at most e (1 - 2 / nc).  The remaining error of w (rounding of
+// qa, of the FMA, and p nc for the reference's p / inc) is below 4 nc 2^-24 <
+// e / (nmax + 1), so |w - rint(w)| <= 1/2 - e (1 - 1 / (nmax + 1)) (qhalf)
+// proves an interior square and holds at the edges.
+//
+// Triangle: f = p rinc - 1/2 - square is within (nmax + 1 + |f|) 2^-23 of the
+// reference's coordinate (unclamped, so the out-of-domain rules are the same
+// tests, see cell_2d_fast); a = f_x - f_y and b = f_x + f_y are decided when
+// the smaller of |a|, |b| exceeds (nmax + 1) 2^-20 (1 + the larger), four
+// times their error.  NaN and infinities fail the test.
+CPAB_HD inline int cell_2d_quick(float px, float py, const Tess &t) {
+    const F2 w = f2_fma({clamp01(px), clamp01(py)}, {t.qa[0], t.qa[1]}, f2_rep(t.qb));
+    const F2 K = f2_add(w, f2_rep(kRoundMagic));
+    const F2 k = f2_add(K, f2_rep(-kRoundMagic));
+    const F2 dw = f2_sub(w, k);
+    const F2 f = f2_sub(f2_fma({px, py}, {t.rinc[0], t.rinc[1]}, f2_rep(-0.5f)), k);
+    const float a = f.x - f.y, b = f.x + f.y;
+    const float lo = fminf(fabsf(a), fabsf(b)), hi = fmaxf(fabsf(a), fabsf(b));
+    const bool ok = fmaxf(fabsf(dw.x), fabsf(dw.y)) <= t.qhalf && lo > fmaf(hi, t.qmargin, t.qmargin);
+    // triangle: 0 (a > 0, b < 0), 1 (a > 0, b > 0), 2 (a < 0, b > 0), 3 (a < 0, b < 0)
+    const int tri = ((float_bits(b) >> 31) + 1) ^ ((float_bits(a) >> 31) & 3);
+    const int c = 4 * ((float_bits(K.x) - kRoundMagicBits) +
+                       (float_bits(K.y) - kRoundMagicBits) * t.nc[0]) + tri;
+    return ok ? c : -1;
+}
+
+// a + b = s + e exactly (Knuth).
+CPAB_HD inline void two_sum(float a, float b, float &s, float &e) {
+    s = CPAB_ADD_RN(a, b);
+    const float bb = CPAB_SUB_RN(s, a);
+    e = CPAB_ADD_RN(CPAB_SUB_RN(a, CPAB_SUB_RN(s, bb)), CPAB_SUB_RN(b, bb));
+}
+
+// a + b - (hi + lo) to within 2^-45 (|a| + |b| + |hi|) and one rounding of the
+// result (which keeps its sign).
+CPAB_HD inline float sum_minus(float a, float b, float hi, float lo) {
+    float s, e, u, v;
+    two_sum(a, b, s, e);
+    two_sum(s, -hi, u, v);
+    return CPAB_ADD_RN(u, CPAB_ADD_RN(v, CPAB_SUB_RN(e, lo)));
+}
+
+// Second tier, for square cells (inc_x == inc_y, Tess::tier2) and points that
+// cell_2d_quick leaves open.  Trajectories that sit on a tie for many steps
+// (zero-boundary domain corners are fixed points up to ~1e-17 drift) come
+// here at every step, and the warp waits for them, so what counts is the
+// length of its dependent chain: it runs in FP32 pairs, not in FP64 (whose
+// latency made one image's forward wait 50 us for its corners, 1 us a step).
+// It follows the reference's branch order (cpab_ops.cpp:57-98) and decides
+// each comparison exactly where that is provable, else returns -1 (FP64
+// replica):
 //  * fx < fy, i.e. rx/ix < ry/iy, and py/iy < px/ix: with one divisor the
 //    correctly rounded double quotients of two distinct floats keep their
 //    order (relative gap >= 2^-24 >> 2^-53), so the float comparison decides;
 //  * 1 - fx < fy: the reference's double evaluation is within 3*2^-53 of
-//    1 - (rx + ry)/ix; T = (ix - rx) - ry in double is within 2^-52 ix of its
-//    exact value, so |T| > 2^-48 ix decides the test by the sign of T;
+//    1 - (rx + ry)/ix; T = (ix - rx) - ry as a float pair is within 2^-46 ix
+//    of its exact value, so |T| > 2^-44 ix decides the test by the sign of T.
+//    With power-of-two cell counts (Tess::pow2) T decides always: closer than
+//    that, rx + ry = ix to 24 bits, so ix - rx - ry is exact, and so is the
+//    reference's 1 - rx nc (rx nc >= 2^-25 there: its last bit is >= 2^-48);
 //  * the out-of-domain rules outside in x and y (cpab_ops.cpp:59-82), e.g.
 //    py/iy - ny > -px/ix: multiplied by ix = iy they compare
 //    D = px + py - ny*iy (or py - px - (ny - nx) ix, px + py - nx ix) with 0.
 //    Each side of the reference's comparison carries at most two roundings
-//    (2^-52 relative); D evaluated in double carries at most 2^-52 of
-//    |px| + |py| + (nx + ny) ix, so |D| above 2^-48 of that decides by its
-//    sign.  Identical evaluations (px == py, nx == ny) compare equal.
-//  * with power-of-two cell counts (Tess::pow2) division by inc is
-//    multiplication by nc, exact in double, so a comparison that the bounds
-//    above leave open is evaluated with the reference's own operations.
+//    (2^-52 relative); D as a float pair carries at most 2^-45 of
+//    |px| + |py| + (nx + ny) ix, so |D| above 2^-44 of that decides by its
+//    sign.  Identical evaluations (px == py, nx == ny) compare equal.  With
+//    power-of-two cell counts what is left is evaluated with the reference's
+//    own double operations (division by inc is multiplication by nc, exact).
 // rx and ry are split_exact's float remainders, equal to the reference's
-// fmod for 0 < p < wlim (and p <= wlim - 1e-9 there, by Tess::tier2).  Called
-// only after cell_2d_fast returned kTie2, i.e. past the band and range checks,
-// so the clamped split is the reference's square.
-static CPAB_HD __noinline__ int cell_2d_tier2(float px, float py, const Tess &t) {
+// fmod for 0 < p < wlim (and p <= wlim - 1e-9 there, by Tess::tier2).
+CPAB_HD inline int cell_2d_tier2(float px, float py, const Tess &t) {
     float fi, ri, fj, rj;
     split_exact(px, t.inc[0], t.rinc[0], fi, ri);
     split_exact(py, t.inc[1], t.rinc[1], fj, rj);
+    // far away, huge or non-finite coordinates: FP64 replica
+    if (!(fabsf(px * t.rinc[0]) < kSplitLimit) || !(fabsf(py * t.rinc[1]) < kSplitLimit))
+        return -1;
     const float ci = fminf(fmaxf(fi, 0.f), t.ncf[0] - 1.f);
     const float cj = fminf(fmaxf(fj, 0.f), t.ncf[1] - 1.f);
+    if (t.band_any &&
+        ((t.band[0] && fi > ci && px < t.wlim[0]) || (t.band[1] && fj > cj && py < t.wlim[1])))
+        return -1;
     const int c = small_float_to_int(4.f * fmaf(cj, t.ncf[0], ci));
-    const double kEps = 3.552713678800501e-15;   // 2^-48
-    const double nix = (double)t.nc[0] * (double)t.inc[0], niy = (double)t.nc[1] * (double)t.inc[1];
-    const double scale = (fabs((double)px) + fabs((double)py)) + (nix + niy);
+    const float kEps = 5.684341886080802e-14f;   // 2^-44
+    const bool left = px <= 0.f, right = px >= t.wlim[0];
+    const bool below = py <= 0.f, above = py >= t.wlim[1];
     int tri;
-    if (px <= 0.f) {
-        if (py <= 0.f) {
+    if ((left || right) && (below || above)) {
+        const float eps = kEps * ((fabsf(px) + fabsf(py)) + (t.nih[0] + t.nih[1]));
+        if (left && below) {
             tri = (py < px) ? 0 : 3;
-        } else if (py >= t.wlim[1]) {                 // py/iy - ny > -px/ix ?
-            const double D = ((double)px + (double)py) - niy;
-            if (fabs(D) > kEps * scale) tri = D > 0.0 ? 2 : 3;
+        } else if (left) {                            // py/iy - ny > -px/ix ?
+            const float D = sum_minus(px, py, t.nih[1], t.nil[1]);
+            if (fabsf(D) > eps) tri = D > 0.f ? 2 : 3;
             else if (t.pow2) tri = ((double)py * t.nc[1] - t.nc[1] > -((double)px * t.nc[0])) ? 2 : 3;
             else return -1;
-        } else {
-            tri = 3;
-        }
-    } else if (px >= t.wlim[0]) {
-        if (py <= 0.f) {                              // -py/iy > px/ix - nx ?
-            const double D = ((double)px + (double)py) - nix;
-            if (fabs(D) > kEps * scale) tri = D < 0.0 ? 0 : 1;
+        } else if (below) {                           // -py/iy > px/ix - nx ?
+            const float D = sum_minus(px, py, t.nih[0], t.nil[0]);
+            if (fabsf(D) > eps) tri = D < 0.f ? 0 : 1;
             else if (t.pow2) tri = (-((double)py * t.nc[1]) > (double)px * t.nc[0] - t.nc[0]) ? 0 : 1;
             else return -1;
-        } else if (py >= t.wlim[1]) {                 // py/iy - ny > px/ix - nx ?
-            if (px == py && t.nc[0] == t.nc[1]) {
-                tri = 1;
-            } else {
-                const double D = ((double)py - (double)px) -
-                                 ((double)t.nc[1] - (double)t.nc[0]) * (double)t.inc[0];
-                if (fabs(D) > kEps * scale) tri = D > 0.0 ? 2 : 1;
-                else if (t.pow2)
-                    tri = ((double)py * t.nc[1] - t.nc[1] > (double)px * t.nc[0] - t.nc[0]) ? 2 : 1;
-                else return -1;
-            }
-        } else {
+        } else if (px == py && t.nc[0] == t.nc[1]) {  // py/iy - ny > px/ix - nx ?
             tri = 1;
+        } else {
+            const float D = sum_minus(py, -px, t.dih, t.dil);
+            if (fabsf(D) > eps) tri = D > 0.f ? 2 : 1;
+            else if (t.pow2)
+                tri = ((double)py * t.nc[1] - t.nc[1] > (double)px * t.nc[0] - t.nc[0]) ? 2 : 1;
+            else return -1;
         }
-    } else if (py <= 0.f) {
+    } else if (left) {
+        tri = 3;
+    } else if (right) {
+        tri = 1;
+    } else if (below) {
         tri = 0;
-    } else if (py >= t.wlim[1]) {
+    } else if (above) {
         tri = 2;
     } else {
-        const double T = ((double)t.inc[0] - (double)ri) - (double)rj;
-        bool s;                                                                   // 1 - fx < fy
-        if (fabs(T) > kEps * (double)t.inc[0]) s = T < 0.0;
-        else if (t.pow2) s = 1.0 - (double)ri * t.nc[0] < (double)rj * t.nc[1];
-        else return -1;
+        const float T = -sum_minus(ri, rj, t.inc[0], 0.f);
+        if (!(fabsf(T) > kEps * t.inc[0]) && !t.pow2) return -1;
+        const bool s = T < 0.f;                                                   // 1 - fx < fy
         tri = (ri < rj) ? (s ? 2 : 3) : (s ? 1 : 0);
     }
     return c + tri;
 }
 
-// FP32 decision of both tiers (-1: the FP64 replica must decide).
+// What cell_2d_quick leaves open: the exact second tier (square cells) or the
+// margins of cell_2d_fast (-1: the FP64 replica must decide).
+CPAB_HD inline int cell_2d_open(float px, float py, const Tess &t) {
+    if (t.tier2) return cell_2d_tier2(px, py, t);
+    return cell_2d_fast(px, py, t);
+}
+
+// FP32 decision of all tiers (-1: the FP64 replica must decide).
 CPAB_HD inline int cell_2d_fp32(float px, float py, const Tess &t) {
-    const int c = cell_2d_fast(px, py, t);
-    if (c >= 0 || c != kTie2 || !t.tier2) return c >= 0 ? c : -1;
-    return cell_2d_tier2(px, py, t);
+    const int c = cell_2d_quick(px, py, t);
+    return c >= 0 ? c : cell_2d_open(px, py, t);
+}
+
+// The cell of a point that cell_2d_quick left open.  Inline: a call costs a warp
+// that waits for a domain corner at every step 0.2 us a step (one 224^2 image
+// 28 against 18 us); the step loops cap their registers instead.
+__device__ __forceinline__ int cell_2d_slow(float px, float py, const Tess &t,
+                                            unsigned long long *ties) {
+    const int c = cell_2d_open(px, py, t);
+    if (c >= 0) return c;
+    if (ties) atomicAdd(ties, 1ull);
+    return cell_2d_exact(px, py, t);
 }
 
 __device__ __forceinline__ int cell_2d(float px, float py, const Tess &t,
                                        unsigned long long *ties) {
-    int c = cell_2d_fast(px, py, t);
-    if (c >= 0) return c;
-    if (c == kTie2 && t.tier2) {
-        c = cell_2d_tier2(px, py, t);
-        if (c >= 0) return c;
-    }
-    if (ties) atomicAdd(ties, 1ull);
-    return cell_2d_exact(px, py, t);
+    const int c = cell_2d_quick(px, py, t);
+    return c >= 0 ? c : cell_2d_slow(px, py, t, ties);
 }
 
 // ------------------------------- 3D ---------------------------------------
@@ -477,6 +635,36 @@ CPAB_HD inline int cell_3d_fast(float p0, float p1, float p2, const Tess &t) {
     return -1;
 }
 
+// First tier of the 3D lookup for power-of-two cell counts (Tess::pow2) and
+// points inside [0, 1] in x and y: inc is 2^-k, so p nc, its floor and the
+// sub-cell coordinates are exact (clamp3 is 1 for x and y, a no-op there), and
+// only the tetrahedron planes need cell_3d_fast's margin.  In a cube at most
+// one of the four tests is positive and every pair of them sums to <= 0, so
+// one test of the smallest |t| replaces the chain of branches.  -1: not
+// decided.
+CPAB_HD inline int cell_3d_quick(float p0, float p1, float p2, const Tess &t) {
+    const F2 u = f2_mul({p0, p1}, {t.ncf[0], t.ncf[1]});
+    const F2 K = f2_floor_magic(u);
+    const F2 r = f2_sub(u, f2_add(K, f2_rep(-kRoundMagic)));
+    const float w = fminf(fmaxf(p2, 0.f), t.clamp3[2]) * t.ncf[2];   // NaN -> 0
+    const float L = floor_magic(w);
+    const float z = CPAB_SUB_RN(w, CPAB_SUB_RN(L, kRoundMagic));
+    // mymin: the index is capped at nc - 1, the remainder is not
+    const int i0 = float_bits(K.x) - kRoundMagicBits, j0 = float_bits(K.y) - kRoundMagicBits;
+    const int k0 = float_bits(L) - kRoundMagicBits;
+    const int i = i0 < t.nc[0] ? i0 : t.nc[0] - 1, j = j0 < t.nc[1] ? j0 : t.nc[1] - 1;
+    const int k = k0 < t.nc[2] ? k0 : t.nc[2] - 1;
+    const bool flip = ((i ^ j ^ k) & 1) != 0;   // the reference's parity rule
+    const float x = flip ? r.y : r.x, y = flip ? CPAB_SUB_RN(1.f, r.x) : r.y;
+    const float s = x + y, d = x - y;
+    const float t1 = z - s, t2 = (s + z) - 2.f, t3 = -d - z, t4 = d - z;
+    const float m = fminf(fminf(fabsf(t1), fabsf(t2)), fminf(fabsf(t3), fabsf(t4)));
+    const bool ok = fminf(p0, p1) >= 0.f && fmaxf(p0, p1) <= 1.f && m > kMargin3;
+    const int sub = t1 > 0.f ? 1 : t2 > 0.f ? 2 : t3 > 0.f ? 3 : t4 > 0.f ? 4 : 0;
+    const int c = 5 * (i + t.nc[0] * (j + t.nc[1] * k)) + sub;
+    return ok ? c : -1;
+}
+
 // Second tier for 3D with power-of-two cell counts (Tess::pow2): inc is then
 // 2^-k, so the reference's sub-cell coordinates r/inc (cpab_ops.cpp:150-155)
 // equal r * nc exactly in double, and its tetrahedron tests
@@ -526,15 +714,24 @@ static CPAB_HD __noinline__ int cell_3d_tier2(float p0, float p1, float p2, cons
     return c;
 }
 
-// FP32-side decision of both 3D tiers (-1: the FP64 replica must decide).
+// FP32-side decision of all 3D tiers (-1: the FP64 replica must decide).
 CPAB_HD inline int cell_3d_fp32(float p0, float p1, float p2, const Tess &t) {
+    if (t.pow2) {
+        const int c = cell_3d_quick(p0, p1, p2, t);
+        if (c >= 0) return c;
+    }
     const int c = cell_3d_fast(p0, p1, p2, t);
     return c >= 0 ? c : cell_3d_tier2(p0, p1, p2, t);
 }
 
 __device__ __forceinline__ int cell_3d(float p0, float p1, float p2, const Tess &t,
                                        unsigned long long *ties) {
-    int c = cell_3d_fast(p0, p1, p2, t);
+    int c;
+    if (t.pow2) {
+        c = cell_3d_quick(p0, p1, p2, t);
+        if (c >= 0) return c;
+    }
+    c = cell_3d_fast(p0, p1, p2, t);
     if (c >= 0) return c;
     c = cell_3d_tier2(p0, p1, p2, t);
     if (c >= 0) return c;
@@ -554,6 +751,38 @@ __device__ __forceinline__ int find_cell(const float (&p)[N], const Tess &t,
     if constexpr (N == 1) return cell_1d(p[0], t);
     else if constexpr (N == 2) return cell_2d(p[0], p[1], t, ties);
     else return cell_3d(p[0], p[1], p[2], t, ties);
+}
+
+// The cells of K points, with one branch for those the first tier leaves open:
+// the K dependent chains up to it overlap.
+template <int N, int K>
+__device__ __forceinline__ void find_cells(const float (&p)[K][N], int (&c)[K], const Tess &t,
+                                           unsigned long long *ties) {
+    if constexpr (N == 2) {
+        int open = 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            c[k] = cell_2d_quick(p[k][0], p[k][1], t);
+            open |= c[k];
+        }
+        if (open < 0) {
+#pragma unroll 1
+            for (int k = 0; k < K; ++k) {
+                float x = p[0][0], y = p[0][1];
+                int v = c[0];
+#pragma unroll
+                for (int j = 1; j < K; ++j)
+                    if (k == j) { x = p[j][0]; y = p[j][1]; v = c[j]; }
+                if (v < 0) v = cell_2d_slow(x, y, t, ties);
+#pragma unroll
+                for (int j = 0; j < K; ++j)
+                    if (k == j) c[j] = v;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; ++k) c[k] = find_cell<N>(p[k], t, ties);
+    }
 }
 
 // --------------------------- device error word ------------------------------

@@ -172,7 +172,8 @@ __device__ void exact_flow_nd(float (&p)[N], const float *tab, const Tess &t,
 
 template <int N>
 __global__ void __launch_bounds__(256)
-    k_integrate_exact(Tess t, const float *__restrict__ points, int broadcast, long long nP,
+    k_integrate_exact(const __grid_constant__ Tess t,
+                      const float *__restrict__ points, int broadcast, long long nP,
                       const float *__restrict__ A, int tiles, float *__restrict__ out,
                       unsigned long long *ties, unsigned *err, unsigned long long *iters) {
     constexpr int P = N * (N + 1);
@@ -248,7 +249,7 @@ cudaError_t launch_integrate_exact(const Tess &t, const float *points, int broad
 // of the warp has used up its time, so all lanes reach every flush.
 template <int N>
 __global__ void __launch_bounds__(128)
-    k_adjoint_exact(Tess t, const float *__restrict__ out, long long nP,
+    k_adjoint_exact(const __grid_constant__ Tess t, const float *__restrict__ out, long long nP,
                     const float *__restrict__ A, int parts, int tiles,
                     const float *__restrict__ gout, float *__restrict__ dpoints,
                     float *__restrict__ partials, unsigned long long *ties, unsigned *err) {

@@ -42,8 +42,9 @@ __device__ __forceinline__ void grid_point(int o, const Geo &g, const float *lin
 }
 
 template <int N, int PPT>
-__global__ void __launch_bounds__(256)
-    k_transform_data(Tess t, int nsteps, Geo g, const float *__restrict__ lin,
+__global__ void __launch_bounds__(256, step_blocks<N>())
+    k_transform_data(const __grid_constant__ Tess t,
+                     int nsteps, Geo g, const float *__restrict__ lin,
                      const float *__restrict__ E, int C, const float *__restrict__ data,
                      float *__restrict__ out, float *__restrict__ grid_out, int tiles,
                      unsigned long long *ties, unsigned *err) {
@@ -66,11 +67,12 @@ __global__ void __launch_bounds__(256)
         }
     }
     for (int s = 0; s < nsteps; ++s) {
+        int c[PPT];
+        find_cells<N, PPT>(p, c, t, ties);
 #pragma unroll
         for (int j = 0; j < PPT; ++j) {
-            int c = find_cell<N>(p[j], t, ties);
             float M[P], y[N];
-            load_cell<N>(tab, c, M);
+            load_cell<N>(tab, c[j], M);
             affine_apply<N>(M, p[j], y);
 #pragma unroll
             for (int r = 0; r < N; ++r) p[j][r] += y[r];
@@ -173,8 +175,9 @@ cudaError_t launch_transform_data(const Tess &t, int nsteps, const float *lin, c
 }
 
 template <int N, int MODE, typename CT, bool GWG>
-__global__ void __launch_bounds__(256)
-    k_transform_data_backward(Tess t, int nsteps, Steps st, Geo g, PreStages pre,
+__global__ void __launch_bounds__(256, step_blocks<N>())
+    k_transform_data_backward(const __grid_constant__ Tess t,
+                              int nsteps, Steps st, Geo g, PreStages pre,
                               const float *__restrict__ lin, const float *__restrict__ table,
                               const float *__restrict__ grid_saved, int C,
                               const float *__restrict__ data, const float *__restrict__ gout,

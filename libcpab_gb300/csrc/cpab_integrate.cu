@@ -23,8 +23,9 @@
 namespace cpab {
 
 template <int N, bool COMP, int PPT>
-__global__ void __launch_bounds__(256)
-    k_integrate(Tess t, int nsteps, const float *__restrict__ points, int broadcast, long long nP,
+__global__ void __launch_bounds__(256, step_blocks<N>())
+    k_integrate(const __grid_constant__ Tess t,
+                int nsteps, const float *__restrict__ points, int broadcast, long long nP,
                 const float *__restrict__ table, int tiles, float *__restrict__ out,
                 int *__restrict__ trace, unsigned long long *ties, unsigned *err) {
     constexpr int P = N * (N + 1);
@@ -47,12 +48,13 @@ __global__ void __launch_bounds__(256)
         for (int r = 0; r < N; ++r) p[j][r] = v ? __ldg(src + r * nP + idx[j]) : 0.5f;
     }
     for (int s = 0; s < nsteps; ++s) {
+        int c[PPT];
+        find_cells<N, PPT>(p, c, t, ties);
 #pragma unroll
         for (int j = 0; j < PPT; ++j) {
-            const int c = find_cell<N>(p[j], t, ties);
-            if (trace && idx[j] < nP) trace[((long long)th * nP + idx[j]) * nsteps + s] = c;
+            if (trace && idx[j] < nP) trace[((long long)th * nP + idx[j]) * nsteps + s] = c[j];
             float M[P], y[N];
-            load_cell<N>(tab, c, M);
+            load_cell<N>(tab, c[j], M);
             affine_apply<N>(M, p[j], y);
 #pragma unroll
             for (int r = 0; r < N; ++r) p[j][r] = COMP ? p[j][r] + y[r] : y[r];
@@ -127,7 +129,8 @@ cudaError_t launch_integrate(const Tess &t, int nsteps, const float *points, int
 }
 
 template <int N>
-__global__ void k_findcellidx(Tess t, const float *__restrict__ points, long long nP,
+__global__ void k_findcellidx(const __grid_constant__ Tess t,
+                              const float *__restrict__ points, long long nP,
                               int *__restrict__ out, unsigned long long *ties) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nP) return;

@@ -38,6 +38,13 @@ bool tuned_get(int kind, const TuneKey &key, LaunchShape *shape);
 void tuned_set(int kind, const TuneKey &key, const LaunchShape &shape);
 void tuned_clear();
 
+// Resident 256-thread blocks per SM that the step-loop kernels are compiled
+// for.  2D: four (64 registers); left alone they take 75-80 for the inlined
+// second lookup tier, which only a few warps run, and lose a block (64 x 224^2
+// backward 1.11 against 0.98 ms).  3D keeps its registers.
+template <int N>
+__host__ __device__ constexpr int step_blocks() { return N == 2 ? 4 : 1; }
+
 // Per-(theta, cell) tables from theta and the basis B [D, d] (fp32):
 // A = B theta, T = expm(dt [A;0]) (rows 0..ndim-1), E = T - I.
 cudaError_t launch_cell_tables(const Tess &t, int nsteps, const float *theta, int n_theta, int d,

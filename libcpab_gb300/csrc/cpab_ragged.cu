@@ -112,7 +112,8 @@ __device__ __forceinline__ Geo series_geo(int L) {
 // integrates PPT points of its warp tile interleaved.
 template <int PPT>
 __global__ void __launch_bounds__(256)
-    k_ragged_forward(Tess t, int nsteps, int S, const long long *__restrict__ off,
+    k_ragged_forward(const __grid_constant__ Tess t,
+                     int nsteps, int S, const long long *__restrict__ off,
                      const int *__restrict__ tile_off, const float *__restrict__ E,
                      const float *__restrict__ values, float *__restrict__ out,
                      unsigned long long *ties, unsigned *err) {
@@ -212,7 +213,8 @@ struct LaneSlotSink {
 
 template <int MODE, typename CT, bool FUSED, bool LS>
 __global__ void __launch_bounds__(256)
-    k_ragged_adjoint(Tess t, int nsteps, Steps st, int S, const long long *__restrict__ off,
+    k_ragged_adjoint(const __grid_constant__ Tess t,
+                     int nsteps, Steps st, int S, const long long *__restrict__ off,
                      const int *__restrict__ tile_off, int ppt, RaggedBwd a,
                      unsigned long long *ties, unsigned *err) {
     constexpr int P = 2;

@@ -20,7 +20,8 @@ namespace cpab {
 
 template <int N, int PPT>
 __global__ void __launch_bounds__(256)
-    k_ragged_points_forward(Tess t, int nsteps, int S, const long long *__restrict__ off,
+    k_ragged_points_forward(const __grid_constant__ Tess t,
+                            int nsteps, int S, const long long *__restrict__ off,
                             const int *__restrict__ tile_off, const float *__restrict__ E,
                             long long total, const float *__restrict__ points,
                             float *__restrict__ out, unsigned long long *ties, unsigned *err) {
@@ -61,11 +62,12 @@ __global__ void __launch_bounds__(256)
                 p[k][r] = (j[k] < L) ? __ldg(points + r * total + base + j[k]) : 0.5f;
         }
         for (int st = 0; st < nsteps; ++st) {
+            int c[PPT];
+            find_cells<N, PPT>(p, c, t, ties);
 #pragma unroll
             for (int k = 0; k < PPT; ++k) {
-                int c = find_cell<N>(p[k], t, ties);
                 float M[P], y[N];
-                load_cell<N>(tab, c, M);
+                load_cell<N>(tab, c[k], M);
                 affine_apply<N>(M, p[k], y);
 #pragma unroll
                 for (int r = 0; r < N; ++r) p[k][r] += y[r];
@@ -98,7 +100,8 @@ __host__ __device__ inline size_t points_adjoint_smem(int nC, int nsteps, int bl
 
 template <int N, int MODE, typename CT>
 __global__ void __launch_bounds__(256, 3)
-    k_ragged_points_adjoint(Tess t, int nsteps, Steps st, int S, const long long *__restrict__ off,
+    k_ragged_points_adjoint(const __grid_constant__ Tess t,
+                            int nsteps, Steps st, int S, const long long *__restrict__ off,
                             const int *__restrict__ tile_off, int ppt,
                             const float *__restrict__ table, long long total,
                             const float *__restrict__ points, const float *__restrict__ gout,
