@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(256, step_blocks<N>())
               unsigned *err) {
     extern __shared__ float4 smem4[];
     __shared__ uint64_t bar;
+    __shared__ int found;
     const int B = blockDim.x, tid = threadIdx.x;
     const int G = t.nC * N * (N + 1);
     const int th = blockIdx.y, part = blockIdx.x;
@@ -73,26 +74,27 @@ __global__ void __launch_bounds__(256, step_blocks<N>())
     const AdjSmem<N, CT> sm =
         carve_adjoint<N, CT, GWG>(reinterpret_cast<float *>(smem4), t.nC, nsteps, gw);
 
+    const float *src = points + (broadcast ? (long long)th * N * nP : 0ll);
+    const PointOrder order = point_order<N>(src, nP, &found);
     if (!adjoint_prologue<N, MODE, CT>(sm, table + (long long)th * G, t.nC, st, &bar, err)) return;
     float *warp_tab = sm.gw + (size_t)(tid >> 5) * round4(G);
-    const float *src = points + (broadcast ? (long long)th * N * nP : 0ll);
 
     for (int tile = part; tile < tiles; tile += parts) {
-        const long long idx = (long long)tile * B + tid;
-        const bool live = idx < nP;
+        const bool live = (long long)tile * B + tid < nP;
+        const long long idx = ordered_point((long long)tile * B + tid, order);
         float p[N], lam[N];
 #pragma unroll
         for (int r = 0; r < N; ++r) p[r] = live ? __ldg(src + r * nP + idx) : 0.5f;
         logged_forward<N, MODE, CT>(sm, t, nsteps, st, p, ties, err);
 #pragma unroll
         for (int r = 0; r < N; ++r) lam[r] = live ? __ldg(gout + ((long long)th * N + r) * nP + idx) : 0.f;
-        reverse_sweep<N, MODE, CT>(sm, nsteps, st, live, lam, warp_tab);
+        reverse_sweep<N, MODE, CT, GWG, false>(sm, nsteps, st, lam, warp_tab);
         if (dpoints && live) {
 #pragma unroll
             for (int r = 0; r < N; ++r) dpoints[((long long)th * N + r) * nP + idx] = lam[r];
         }
     }
-    adjoint_epilogue<N, CT>(sm, t.nC, partials + ((long long)th * parts + part) * G);
+    adjoint_epilogue<N, CT, GWG>(sm, t.nC, partials + ((long long)th * parts + part) * G);
 }
 
 // ------------------------------ planning -------------------------------------
@@ -110,8 +112,9 @@ static bool plan_t(const Tess &t, int nsteps, long long nP, int n_theta, Adjoint
                               &global_gw, &smem, &per_sm, sh.block, sh.staging))
         return false;
     const long long tiles = (nP + block - 1) / block;
-    const long long target = 2ll * num_sms() * per_sm;
-    long long parts = sh.parts > 0 ? sh.parts : (target + n_theta - 1) / n_theta;
+    long long parts = sh.parts > 0 ? sh.parts
+                                   : adjoint_parts(tiles, n_theta, (long long)num_sms() * per_sm,
+                                                   t.nC * N * (N + 1), global_gw ? 4.0 : 1e9);
     if (parts > tiles) parts = tiles;
     if (parts < 1) parts = 1;
     plan->block = block;

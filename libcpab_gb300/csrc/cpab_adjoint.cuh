@@ -2,6 +2,7 @@
 // fused transform_data backward (cpab_fused.cu).  The scheme is described at
 // the top of cpab_adjoint.cu.
 #pragma once
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -158,10 +159,8 @@ __device__ __forceinline__ void load_dtab(const float *dtab, int c, float (&D)[N
 // lambda_{n+1}.  Both modes accumulate the same outer product; the mode-0
 // cell gradient G_c is a fixed linear map of S_c applied in k_finalize.
 template <int N>
-__device__ __forceinline__ void adjoint_step(const float *dtab, int c, const float (&p)[N],
+__device__ __forceinline__ void adjoint_step(const float (&D)[N * N], const float (&p)[N],
                                              float (&lam)[N], float (&acc)[N * (N + 1)]) {
-    float D[N * N];
-    load_dtab<N>(dtab, c, D);
 #pragma unroll
     for (int r = 0; r < N; ++r) {
 #pragma unroll
@@ -246,6 +245,34 @@ inline bool adjoint_shape(K kern_shared, K kern_global, int nC, int nsteps, int 
     return best > 0;
 }
 
+// Host: CTAs per theta (or image), each taking every parts-th of its `tiles`
+// tiles, for n of them on a GPU that holds `resident` CTAs.  In units of a
+// tile the launch lasts about the average load of a resident slot (or, within
+// one wave, one CTA, `own` tiles), plus 0.17 own for the uneven end (fitted to
+// 9 .. 196 CTAs per image of 64 x 224^2), plus the setup of each CTA's tables of
+// G floats.  Small tables are cheap, so most launches take one tile per CTA: 16
+// images of 196 tiles 258 us, against 336 us with two waves of CTAs of up to 3
+// tiles (the earlier rule), 64 images 921 against 1,003 us.
+// max_waves bounds the CTAs (tables in global memory take space for each).
+inline long long adjoint_parts(long long tiles, long long n, long long resident, int G,
+                               double max_waves) {
+    const double setup = 1e-4 * G;
+    const long long most =
+        std::max(1ll, std::min(tiles, (long long)(max_waves * (double)resident / (double)n) + 1));
+    long long best = 1;
+    double least = 0.0;
+    for (long long p = 1; p <= most; p = p < 512 ? p + 1 : p + p / 64) {
+        const double own = (double)((tiles + p - 1) / p), waves = (double)(n * p) / (double)resident;
+        const double load = (double)(n * tiles) / (double)resident;
+        const double cost = std::max(load, waves <= 1.0 ? own : 0.0) + 0.17 * own + waves * setup;
+        if (p == 1 || cost < least) {
+            best = p;
+            least = cost;
+        }
+    }
+    return best;
+}
+
 // Host: launch plans are computed once per problem shape and device (the
 // occupancy queries behind a plan cost tens of microseconds, on the critical
 // path of an eager training step).
@@ -310,6 +337,119 @@ __device__ __forceinline__ AdjSmem<N, CT> carve_adjoint(float *base, int nC, int
     return s;
 }
 
+// dst += v in the warp's table.  In global memory a fire-and-forget reduction:
+// its element gets one addition per flush, flushes are ordered by __syncwarp,
+// so the order of the sum is fixed all the same and nobody waits for a load.
+template <bool GWG>
+__device__ __forceinline__ void table_add(float *dst, float v) {
+    if constexpr (GWG) atomicAdd(dst, v);
+    else *dst += v;
+}
+
+// Sums of v[0..P) over the warp by recursive halving: at each round a lane
+// keeps half of the values it holds and gives the other half to its partner,
+// so P = 6 (padded to 8) takes 9 shuffles instead of 30.  Afterwards lane l
+// holds, in v[0], the sum of value sum_index(l), the same in each lane that
+// shares the index; the order of the additions is fixed.
+template <int W, int P>
+__device__ __forceinline__ void halve(float (&v)[P], int xor_lane, bool up) {
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+        const float send = up ? v[i] : v[i + W], keep = up ? v[i + W] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, xor_lane);
+    }
+}
+
+__host__ __device__ constexpr int pad_pow2(int P) { return P <= 2 ? 2 : P <= 8 ? 8 : 16; }
+
+// Index of the value whose sum lane l holds (>= P: padding).
+template <int P>
+__device__ __forceinline__ int sum_index(int lane) {
+    if constexpr (pad_pow2(P) == 16) return lane >> 1;
+    else if constexpr (pad_pow2(P) == 8) return lane >> 2;
+    else return lane >> 4;
+}
+
+template <int P>
+__device__ __forceinline__ float warp_sums(const float (&acc)[P], bool in) {
+    constexpr int W = pad_pow2(P);
+    const int lane = threadIdx.x & 31;
+    float v[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) v[i] = (i < P && in) ? acc[i < P ? i : 0] : 0.f;
+    halve<W / 2>(v, 16, lane & 16);
+    if constexpr (W >= 8) {
+        halve<W / 4>(v, 8, lane & 8);
+        halve<W / 8>(v, 4, lane & 4);
+    }
+    if constexpr (W >= 16) halve<1>(v, 2, lane & 2);
+#pragma unroll
+    for (int d = 16 / W; d > 0; d >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], d);
+    return v[0];
+}
+
+// Add the accumulators of the lanes that leave their cell at this step into
+// the warp's cell table, for warps of neighbouring points (called by all lanes
+// of the warp).  A lane that leaves its cell alone adds its sums itself.  Lanes
+// that leave the same cell together, as neighbours that cross a face do, are
+// summed first: up to four of a kind one after the other into their lowest
+// lane, all cells at once (15 instructions per lane of the largest group),
+// else one cell after the other by warp_sums (50 instructions per cell).  Every
+// table element so receives at most one addition per step, in step order, and
+// the summation order depends only on the inputs: the sums are reproducible.
+// [8,8] on a 512^2 meshgrid, adjoint kernel: 7.1 ms with flush_scattered, 6.4 ms
+// with this, 5.1 ms on patches (PointOrder).
+constexpr int kChainLanes = 4;
+
+template <int P, bool GWG>
+__device__ __forceinline__ void flush_neighbours(bool change, int cell, const float (&acc)[P],
+                                                 float *warp_tab) {
+    const int lane = threadIdx.x & 31;
+    const unsigned grp = __match_any_sync(0xffffffffu, change ? cell : -1 - lane);
+    const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)__popc(grp));
+    if (most <= kChainLanes) {
+        float sum[P];
+#pragma unroll
+        for (int i = 0; i < P; ++i) sum[i] = acc[i];
+        unsigned rest = grp & (grp - 1u);        // the other members, lowest first
+#pragma unroll 1
+        for (int k = 1; k < most; ++k) {
+            const int src = rest ? __ffs(rest) - 1 : lane;
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                const float u = __shfl_sync(0xffffffffu, acc[i], src);
+                if (rest) sum[i] += u;
+            }
+            rest &= rest - 1u;
+        }
+        if (change && lane == __ffs(grp) - 1) {
+            float *dst = warp_tab + cell * P;
+#pragma unroll
+            for (int i = 0; i < P; ++i) table_add<GWG>(dst + i, sum[i]);
+        }
+    } else {
+        const bool alone = (grp & (grp - 1u)) == 0u;
+        unsigned todo = __ballot_sync(0xffffffffu, change && !alone);
+        if (change && alone) {
+            float *dst = warp_tab + cell * P;
+#pragma unroll
+            for (int i = 0; i < P; ++i) table_add<GWG>(dst + i, acc[i]);
+        }
+#pragma unroll 1
+        while (todo) {
+            const int first = __ffs(todo) - 1;
+            const unsigned g = __shfl_sync(0xffffffffu, grp, first);
+            const int c = __shfl_sync(0xffffffffu, cell, first);
+            const float v = warp_sums<P>(acc, (g >> lane) & 1u);
+            const int i = sum_index<P>(lane);
+            if (i < P && (lane & (32 / pad_pow2(P) - 1)) == 0)
+                table_add<GWG>(warp_tab + c * P + i, v);
+            todo &= ~g;
+        }
+    }
+    __syncwarp();
+}
+
 // Sum each contiguous lane run [lo, hi] of sum[] into lane lo (five fixed
 // shuffle rounds) and add it there.  All lanes of m call it; runs lie in m.
 template <int P>
@@ -329,8 +469,10 @@ __device__ __forceinline__ void add_runs(unsigned m, int lo, int hi, float (&sum
     }
 }
 
-// Add the accumulators of the lanes in m (the lanes leaving a cell at this
-// step; called by exactly those lanes) into the warp's cell table.  Lanes that
+// The same for warps of scattered points, called by exactly the lanes in m that
+// leave a cell at this step: the largest group decides how all are summed, which
+// is cheaper where groups are few and small (1,024 sets of random points 2.54
+// against 2.65 ms).  Lanes that
 // leave the same cell at the same step are first summed into their lowest
 // lane (a fixed shuffle tree when every group is a contiguous run of more than
 // four lanes, else a lane-order chain), so every table element receives at
@@ -338,7 +480,7 @@ __device__ __forceinline__ void add_runs(unsigned m, int lo, int hi, float (&sum
 // on the inputs: the sums are reproducible.  In the common case (no two lanes
 // share a cell) all lanes add in one pass.
 template <int P>
-__device__ __forceinline__ void flush_cells(unsigned m, int cell, const float (&acc)[P],
+__device__ __forceinline__ void flush_scattered(unsigned m, int cell, const float (&acc)[P],
                                             float *warp_tab) {
     const int lane = threadIdx.x & 31;
     float *dst = warp_tab + cell * P;
@@ -384,7 +526,7 @@ __device__ __forceinline__ void warp_flush(bool flush, int cell, const float (&a
                                            float *warp_tab) {
     const unsigned m = __ballot_sync(0xffffffffu, flush);
     if (m) {
-        if (flush) flush_cells<P>(m, cell, acc, warp_tab);
+        if (flush) flush_scattered<P>(m, cell, acc, warp_tab);
         __syncwarp();
     }
 }
@@ -395,7 +537,7 @@ __device__ __forceinline__ void warp_flush(bool flush, int cell, const float (&a
 // Then every lane takes part in a fixed five-round shuffle tree over its run
 // (non-flushing lanes add zeros) and the run's lowest lane adds the sum if
 // any lane of the run flushes: the same one-add-per-element-per-step
-// discipline as flush_cells, without match.any.  Unsorted warps use
+// discipline as flush_scattered, without match.any.  Unsorted warps use
 // warp_flush.  Called by all lanes of the warp.
 template <int P>
 __device__ __forceinline__ void warp_flush_1d(bool flush, int cell, const float (&acc)[P],
@@ -434,37 +576,49 @@ __device__ __forceinline__ void warp_flush_1d(bool flush, int cell, const float 
 }
 
 // Where reverse_sweep puts a lane's accumulated dL/dA of a cell when the lane
-// leaves it: the warp's cell table, through warp_flush / warp_flush_1d
-// (called by all lanes of the warp).
-template <int N>
+// leaves it: the warp's cell table.  changed() is called by all lanes of the
+// warp with the ballot of the lanes that leave their cell, not zero.
+// SCATTERED: the warp's points are in no order that this code knows of.
+template <int N, bool GWG, bool SCATTERED>
 struct WarpTabSink {
+    static constexpr bool kWarp = true;   // changed() is a warp-wide call
     float *warp_tab;
     template <int P>
-    __device__ __forceinline__ void operator()(bool flush, int cell,
-                                               const float (&acc)[P]) const {
-        if constexpr (N == 1) warp_flush_1d<P>(flush, cell, acc, warp_tab);
-        else warp_flush<P>(flush, cell, acc, warp_tab);
+    __device__ __forceinline__ void changed(unsigned m, bool change, int cell,
+                                            const float (&acc)[P]) const {
+        if constexpr (N == 1) {
+            warp_flush_1d<P>(change, cell, acc, warp_tab);
+        } else if constexpr (SCATTERED) {
+            if (change) flush_scattered<P>(m, cell, acc, warp_tab);
+            __syncwarp();
+        } else {
+            flush_neighbours<P, GWG>(change, cell, acc, warp_tab);
+        }
     }
 };
 
 // Reverse sweep of one trajectory whose cells are logged in cl and whose
-// checkpoints are in ck; lam holds dL/dp_N on entry and dL/dp_0 on exit.
+// checkpoints are in ck; lam holds dL/dp_N on entry (0 for a lane without a
+// point, whose sums are then zeros) and dL/dp_0 on exit.
 // Each segment's positions are rebuilt from its checkpoint with the logged
 // cells (no lookups) into pb, then walked backwards.  The loops are not
-// unrolled: the body stays small enough for the instruction cache.
-// Executed by all lanes of the warp (uniform trip counts); sink(flush, cell,
-// acc) receives each lane's sum over a run of steps in one cell.
+// unrolled: the body stays small enough for the instruction cache (unrolled by
+// five, with the positions in registers, it ran 18 % fewer instructions and
+// took 35 % longer at [8,8], 18 % at [4,4,4]).  A lane reloads the propagator
+// only where it enters another cell.
+// Executed by all lanes of the warp (uniform trip counts); sink receives each
+// lane's sum over a run of steps in one cell.
 template <int N, int MODE, typename CT, typename Sink>
 __device__ __forceinline__ void reverse_sweep_to(const AdjSmem<N, CT> &sm, int nsteps,
-                                                 const Steps &st, bool live, float (&lam)[N],
-                                                 Sink &sink) {
+                                                 const Steps &st, float (&lam)[N], Sink &sink) {
     constexpr int P = N * (N + 1);
     const int B = blockDim.x, tid = threadIdx.x;
     const int nseg = (nsteps + kSeg - 1) / kSeg;
-    float acc[P];
+    float acc[P], D[N * N];
 #pragma unroll
     for (int i = 0; i < P; ++i) acc[i] = 0.f;
-    int gcell = -1;
+    int gcell = (int)sm.cl[(nsteps - 1) * B + tid];
+    load_dtab<N>(sm.dtab, gcell, D);
     for (int seg = nseg - 1; seg >= 0; --seg) {
         const int n0 = seg * kSeg;
         const int len = min(kSeg, nsteps - n0);
@@ -482,27 +636,31 @@ __device__ __forceinline__ void reverse_sweep_to(const AdjSmem<N, CT> &sm, int n
         for (int s = len - 1; s >= 0; --s) {
             const int c = (int)sm.cl[(n0 + s) * B + tid];
             const bool change = c != gcell;
-            sink(change && gcell >= 0 && live, gcell, acc);
-            if (change) {
-                gcell = c;
+            const unsigned m = Sink::kWarp ? __ballot_sync(0xffffffffu, change) : change;
+            if (m) {
+                sink.changed(m, change, gcell, acc);
+                if (change) {
+                    gcell = c;
 #pragma unroll
-                for (int i = 0; i < P; ++i) acc[i] = 0.f;
+                    for (int i = 0; i < P; ++i) acc[i] = 0.f;
+                    load_dtab<N>(sm.dtab, c, D);
+                }
             }
             float p[N];
 #pragma unroll
             for (int r = 0; r < N; ++r) p[r] = sm.pb[(s * N + r) * B + tid];
-            adjoint_step<N>(sm.dtab, c, p, lam, acc);
+            adjoint_step<N>(D, p, lam, acc);
         }
     }
-    sink(gcell >= 0 && live, gcell, acc);
+    sink.changed(0xffffffffu, true, gcell, acc);
 }
 
-template <int N, int MODE, typename CT>
+template <int N, int MODE, typename CT, bool GWG, bool SCATTERED>
 __device__ __forceinline__ void reverse_sweep(const AdjSmem<N, CT> &sm, int nsteps,
-                                              const Steps &st, bool live, float (&lam)[N],
+                                              const Steps &st, float (&lam)[N],
                                               float *warp_tab) {
-    WarpTabSink<N> sink{warp_tab};
-    reverse_sweep_to<N, MODE, CT>(sm, nsteps, st, live, lam, sink);
+    WarpTabSink<N, GWG, SCATTERED> sink{warp_tab};
+    reverse_sweep_to<N, MODE, CT>(sm, nsteps, st, lam, sink);
 }
 
 // Sweep with the arithmetic of k_integrate's compensated path,
@@ -541,6 +699,61 @@ __device__ __forceinline__ void logged_forward(const AdjSmem<N, CT> &sm, const T
     }
 }
 
+// Order of a theta's points over the threads of the adjoint.  The points of a
+// meshgrid (the first axis fastest, uniform_meshgrid's order) are taken in
+// patches of 8 x 4, 4 x 8 or 16 x 2 points per warp instead of 32 along a row:
+// the lanes then cross a cell boundary at nearly the same step, so the warp
+// flushes its cell sums at fewer steps (flush_neighbours).  The length of a row
+// is read off the points: it is the number of leading points that share their
+// second coordinate.  Any points may be passed, this is a permutation of them
+// whatever they are.
+struct PointOrder {
+    int row, wide, shift;   // row length (0: in order), patch width and log2 of it
+};
+
+constexpr int kMaxRow = 1024;   // rows looked for (four reads of a 256-thread block)
+
+// Called by all threads of the block; `found` is shared.
+template <int N>
+__device__ __forceinline__ PointOrder point_order(const float *points, long long nP, int *found) {
+    PointOrder o = {0, 32, 5};
+    if constexpr (N >= 2) {
+        if (nP < 64 || nP >= (1ll << 31)) return o;
+        if (threadIdx.x == 0) *found = kMaxRow + 1;
+        __syncthreads();
+        const float *y = points + nP;
+        const float y0 = __ldg(y);
+        const int most = (int)min(nP, (long long)kMaxRow + 1);
+        int row = kMaxRow + 1;
+        for (int i = 1 + threadIdx.x; i - (int)threadIdx.x < most; i += blockDim.x) {
+            if (i < most && __ldg(y + i) != y0) atomicMin(found, i);
+            __syncthreads();
+            row = *found;
+            __syncthreads();
+            if (row <= kMaxRow) break;
+        }
+        if (row > kMaxRow || nP % row) return o;
+        const int rows = (int)(nP / row);
+        if (row % 8 == 0 && rows % 4 == 0) o.shift = 3;
+        else if (row % 4 == 0 && rows % 8 == 0) o.shift = 2;
+        else if (row % 16 == 0 && rows % 2 == 0) o.shift = 4;
+        else return o;
+        o.row = row;
+        o.wide = 1 << o.shift;
+    }
+    return o;
+}
+
+// Index of the point of thread v.
+__device__ __forceinline__ long long ordered_point(long long v, const PointOrder &o) {
+    if (!o.row) return v;
+    const unsigned w = (unsigned)(v >> 5), lane = (unsigned)v & 31u;
+    const unsigned per = (unsigned)o.row >> o.shift;
+    const unsigned band = w / per, col = w - band * per;
+    const unsigned r = band * (32u >> o.shift) + (lane >> o.shift);
+    return (long long)r * o.row + col * o.wide + (lane & (o.wide - 1u));
+}
+
 // Kernel prologue: stage the cell table, build the propagators and clear the
 // per-warp tables.  Returns false (block exits) if staging failed.
 template <int N, int MODE, typename CT>
@@ -558,14 +771,17 @@ __device__ __forceinline__ bool adjoint_prologue(const AdjSmem<N, CT> &sm, const
 
 // Kernel epilogue: write this CTA's partial (per-warp tables summed in warp
 // order).
-template <int N, typename CT>
+template <int N, typename CT, bool GWG>
 __device__ __forceinline__ void adjoint_epilogue(const AdjSmem<N, CT> &sm, int nC, float *dst) {
     constexpr int P = N * (N + 1);
     const int B = blockDim.x, W = B / 32, G = nC * P, Gr = round4(G);
     __syncthreads();
     for (int i = threadIdx.x; i < G; i += B) {
         float s = 0.f;
-        for (int w = 0; w < W; ++w) s += sm.gw[(size_t)w * Gr + i];
+        for (int w = 0; w < W; ++w) {
+            const float *q = sm.gw + (size_t)w * Gr + i;
+            s += GWG ? __ldcg(q) : *q;   // the reductions are in L2
+        }
         dst[i] = s;
     }
 }

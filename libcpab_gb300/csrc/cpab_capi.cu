@@ -534,10 +534,9 @@ size_t cpab_transform_data_backward_workspace(int ndim, const int *nc, int nstep
     if (make_tess(ndim, nc, &t) || check_steps(nsteps) || check_sizes(ndim, outsize, "outsize"))
         return 0;
     if (nb <= 0 || (!grad_mode_ok(mode))) return 0;
-    long long nP = 1;
-    for (int j = 0; j < ndim; ++j) nP *= outsize[j];
+    const long long threads = transform_data_backward_threads(ndim, outsize);
     AdjointPlan plan;
-    if (!plan_transform_data_backward(t, nsteps, mode, nP, nb, &plan)) {
+    if (!plan_transform_data_backward(t, nsteps, mode, threads, nb, &plan)) {
         fail(CPAB_ERR_UNSUPPORTED, "tessellation/nsteps too large for the adjoint kernel");
         return 0;
     }
@@ -571,10 +570,9 @@ static int td_backward(int ndim, const int *nc, int nsteps, int mode, const floa
     if (mode == CPAB_GRAD_EXACT && !E) return fail(CPAB_ERR_ARGUMENT, "exact mode needs E");
     if (mode != CPAB_GRAD_EXACT && !grid_saved)
         return fail(CPAB_ERR_ARGUMENT, "reference mode needs grid_saved");
-    long long nP = 1;
-    for (int j = 0; j < ndim; ++j) nP *= outsize[j];
+    const long long threads = transform_data_backward_threads(ndim, outsize);
     AdjointPlan plan;
-    if (!plan_transform_data_backward(t, nsteps, mode, nP, nb, &plan, force))
+    if (!plan_transform_data_backward(t, nsteps, mode, threads, nb, &plan, force))
         return fail(CPAB_ERR_UNSUPPORTED, "tessellation/nsteps too large for the adjoint kernel");
     const size_t need = plan.ws_floats() * sizeof(float);
     if (!workspace || workspace_bytes < need)
@@ -1491,10 +1489,9 @@ int cpab_transform_data_backward_tune(int ndim, const int *nc, int nsteps, int m
     if ((rc = refuse_capture(s, "cpab_transform_data_backward_tune"))) return rc;
     LaunchShape fs;
     if (force && (rc = check_adjoint_shape(fs = get_shape(force), ndim))) return rc;
-    long long nP = 1;
-    for (int j = 0; j < ndim; ++j) nP *= outsize[j];
+    const long long threads = transform_data_backward_threads(ndim, outsize);
     auto plan = [&](const LaunchShape &sh, AdjointPlan *pl) {
-        return plan_transform_data_backward(t, nsteps, mode, nP, nb, pl, &sh);
+        return plan_transform_data_backward(t, nsteps, mode, threads, nb, pl, &sh);
     };
     size_t ws_max = 0;
     std::vector<LaunchShape> cands = adjoint_candidates(ndim, plan, &ws_max);
@@ -1511,7 +1508,7 @@ int cpab_transform_data_backward_tune(int ndim, const int *nc, int nsteps, int m
                            size, basis, d, grad_out, ddata, dtheta, ws.p, ws.bytes, nullptr,
                            stream, nullptr, &sh);
     };
-    return tune_family(kTuneFusedBackward, tune_key(t, nsteps, mode, nP, nb, 0), cands,
+    return tune_family(kTuneFusedBackward, tune_key(t, nsteps, mode, threads, nb, 0), cands,
                        force ? &fs : nullptr, s, run, shape, best_ms);
 }
 

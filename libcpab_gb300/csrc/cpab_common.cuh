@@ -186,6 +186,7 @@ struct F2 {
         return d;                                                                                 \
     }
 CPAB_F2_OP2(f2_add, "add.rn.f32x2")
+CPAB_F2_OP2(f2_sub, "sub.rn.f32x2")
 CPAB_F2_OP2(f2_mul, "mul.rn.f32x2")
 CPAB_F2_OP2(f2_add_rd, "add.rm.f32x2")
 #undef CPAB_F2_OP2
@@ -199,12 +200,11 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
 }
 #else
 inline F2 f2_add(F2 a, F2 b) { return {a.x + b.x, a.y + b.y}; }
+inline F2 f2_sub(F2 a, F2 b) { return {a.x - b.x, a.y - b.y}; }
 inline F2 f2_mul(F2 a, F2 b) { return {a.x * b.x, a.y * b.y}; }
 inline F2 f2_fma(F2 a, F2 b, F2 c) { return {fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
 #endif
 CPAB_HD inline F2 f2_rep(float v) { return {v, v}; }
-// a - b (b negated inside an FMA: exact)
-CPAB_HD inline F2 f2_sub(F2 a, F2 b) { return f2_fma(b, f2_rep(-1.f), a); }
 
 // kRoundMagic + floor(x) for |x| < 2^22 (one add rounded towards -infinity;
 // the sum's ulp is 1)
@@ -381,18 +381,18 @@ CPAB_HD inline int cell_2d_fast(float px, float py, const Tess &t) {
 // e / (nmax + 1), so |w - rint(w)| <= 1/2 - e (1 - 1 / (nmax + 1)) (qhalf)
 // proves an interior square and holds at the edges.
 //
-// Triangle: f = p rinc - 1/2 - square is within (nmax + 1 + |f|) 2^-23 of the
+// Triangle: f = p rinc - square is within (nmax + 1 + |f|) 2^-23 of the
 // reference's coordinate (unclamped, so the out-of-domain rules are the same
-// tests, see cell_2d_fast); a = f_x - f_y and b = f_x + f_y are decided when
-// the smaller of |a|, |b| exceeds (nmax + 1) 2^-20 (1 + the larger), four
-// times their error.  NaN and infinities fail the test.
+// tests, see cell_2d_fast); a = f_x - f_y and b = f_x + f_y - 1 are decided
+// when the smaller of |a|, |b| exceeds (nmax + 1) 2^-20 (1 + the larger), at
+// least twice their error (|f_x| + |f_y| <= |a| + |b| + 1).  NaN and infinities fail the test.
 CPAB_HD inline int cell_2d_quick(float px, float py, const Tess &t) {
     const F2 w = f2_fma({clamp01(px), clamp01(py)}, {t.qa[0], t.qa[1]}, f2_rep(t.qb));
     const F2 K = f2_add(w, f2_rep(kRoundMagic));
-    const F2 k = f2_add(K, f2_rep(-kRoundMagic));
+    const F2 k = f2_sub(K, f2_rep(kRoundMagic));
     const F2 dw = f2_sub(w, k);
-    const F2 f = f2_sub(f2_fma({px, py}, {t.rinc[0], t.rinc[1]}, f2_rep(-0.5f)), k);
-    const float a = f.x - f.y, b = f.x + f.y;
+    const F2 f = f2_sub(f2_mul({px, py}, {t.rinc[0], t.rinc[1]}), k);
+    const float a = f.x - f.y, b = (f.x + f.y) - 1.f;
     const float lo = fminf(fabsf(a), fabsf(b)), hi = fmaxf(fabsf(a), fabsf(b));
     const bool ok = fmaxf(fabsf(dw.x), fabsf(dw.y)) <= t.qhalf && lo > fmaf(hi, t.qmargin, t.qmargin);
     // triangle: 0 (a > 0, b < 0), 1 (a > 0, b > 0), 2 (a < 0, b > 0), 3 (a < 0, b < 0)
@@ -645,7 +645,7 @@ CPAB_HD inline int cell_3d_fast(float p0, float p1, float p2, const Tess &t) {
 CPAB_HD inline int cell_3d_quick(float p0, float p1, float p2, const Tess &t) {
     const F2 u = f2_mul({p0, p1}, {t.ncf[0], t.ncf[1]});
     const F2 K = f2_floor_magic(u);
-    const F2 r = f2_sub(u, f2_add(K, f2_rep(-kRoundMagic)));
+    const F2 r = f2_sub(u, f2_sub(K, f2_rep(kRoundMagic)));
     const float w = fminf(fmaxf(p2, 0.f), t.clamp3[2]) * t.ncf[2];   // NaN -> 0
     const float L = floor_magic(w);
     const float z = CPAB_SUB_RN(w, CPAB_SUB_RN(L, kRoundMagic));

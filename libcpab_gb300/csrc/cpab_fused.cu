@@ -41,6 +41,56 @@ __device__ __forceinline__ void grid_point(int o, const Geo &g, const float *lin
     }
 }
 
+// Order of an image's points over the threads of the backward (2D, 3D): a warp
+// takes a patch of 4 x 8 points (the last two axes) instead of 32 points along
+// the last axis.  The lanes then cross a cell boundary at nearly the same step,
+// so the warp flushes its cell sums at fewer steps; loads and stores stay whole
+// 32-byte sectors.  Patches cut by the edge leave lanes without a point: where
+// that would cost more than 1/16 of the threads the points are taken in order.
+struct Patch {
+    int on;
+    FastDiv dz, dy;   // patches along the last axis and the one before it
+};
+
+static Patch make_patch(int ndim, const int *outsize, long long *threads) {
+    Patch q = {};
+    long long nP = 1, padded = 32;
+    for (int j = 0; j < ndim; ++j) nP *= outsize[j];
+    *threads = nP;
+    if (ndim < 2 || nP == 0) return q;
+    const int nz = (outsize[ndim - 1] + 7) / 8, ny = (outsize[ndim - 2] + 3) / 4;
+    padded *= (long long)nz * ny * (ndim == 3 ? outsize[0] : 1);
+    if (padded > nP + nP / 16 || padded >= (1ll << 31)) return q;
+    *threads = padded;
+    q.on = 1;
+    q.dz = make_fastdiv((unsigned)nz);
+    q.dy = make_fastdiv((unsigned)ny);
+    return q;
+}
+
+long long transform_data_backward_threads(int ndim, const int *outsize) {
+    long long n;
+    make_patch(ndim, outsize, &n);
+    return n;
+}
+
+// Output index of thread v, or -1 for a thread without a point.
+template <int N>
+__device__ __forceinline__ int patch_point(int v, const Patch &q, const Geo &g) {
+    if constexpr (N >= 2) {
+        if (q.on) {
+            const unsigned w = (unsigned)v >> 5, lane = v & 31;
+            const unsigned wz = fast_div(w, q.dz), zc = w - wz * q.dz.d;
+            const unsigned x = fast_div(wz, q.dy), yc = wz - x * q.dy.d;
+            const int z = zc * 8 + (lane & 7), y = yc * 4 + (lane >> 3);
+            if (z >= g.outsize[N - 1] || y >= g.outsize[N - 2] || (int)x >= (N == 3 ? g.outsize[0] : 1))
+                return -1;
+            return ((int)x * g.outsize[N - 2] + y) * g.outsize[N - 1] + z;
+        }
+    }
+    return v < g.nP ? v : -1;
+}
+
 template <int N, int PPT>
 __global__ void __launch_bounds__(256, step_blocks<N>())
     k_transform_data(const __grid_constant__ Tess t,
@@ -177,7 +227,7 @@ cudaError_t launch_transform_data(const Tess &t, int nsteps, const float *lin, c
 template <int N, int MODE, typename CT, bool GWG>
 __global__ void __launch_bounds__(256, step_blocks<N>())
     k_transform_data_backward(const __grid_constant__ Tess t,
-                              int nsteps, Steps st, Geo g, PreStages pre,
+                              int nsteps, Steps st, Geo g, Patch patch, PreStages pre,
                               const float *__restrict__ lin, const float *__restrict__ table,
                               const float *__restrict__ grid_saved, int C,
                               const float *__restrict__ data, const float *__restrict__ gout,
@@ -197,8 +247,8 @@ __global__ void __launch_bounds__(256, step_blocks<N>())
     float *warp_tab = sm.gw + (size_t)(tid >> 5) * round4(G);
 
     for (int tile = part; tile < tiles; tile += parts) {
-        const int o = tile * B + tid;
-        const bool live = o < g.nP;
+        const int o = patch_point<N>(tile * B + tid, patch, g);
+        const bool live = o >= 0;
         float p[N], pN[N], lam[N];
         if (live) grid_point<N>(o, g, lin, p);
         else {
@@ -232,13 +282,13 @@ __global__ void __launch_bounds__(256, step_blocks<N>())
         }
 #pragma unroll
         for (int r = 0; r < N; ++r) lam[r] = gf[r] * (float)(g.size[r] - 1);
-        reverse_sweep<N, MODE, CT>(sm, nsteps, st, live, lam, warp_tab);
+        reverse_sweep<N, MODE, CT, GWG, false>(sm, nsteps, st, lam, warp_tab);
     }
-    adjoint_epilogue<N, CT>(sm, t.nC, partials + ((long long)b * parts + part) * G);
+    adjoint_epilogue<N, CT, GWG>(sm, t.nC, partials + ((long long)b * parts + part) * G);
 }
 
 template <int N, int MODE, typename CT>
-static bool plan_td_t(const Tess &t, int nsteps, long long nP, int nb, AdjointPlan *plan,
+static bool plan_td_t(const Tess &t, int nsteps, long long threads, int nb, AdjointPlan *plan,
                       const LaunchShape &sh) {
     int block = 0, per_sm = 0;
     bool global_gw = false;
@@ -249,9 +299,10 @@ static bool plan_td_t(const Tess &t, int nsteps, long long nP, int nb, AdjointPl
     if (!adjoint_shape<N, CT>(k_transform_data_backward<N, MODE, CT, false>, kg, t.nC, nsteps,
                               &block, &global_gw, &smem, &per_sm, sh.block, sh.staging))
         return false;
-    const long long tiles = (nP + block - 1) / block;
-    const long long target = 2ll * num_sms() * per_sm;
-    long long parts = sh.parts > 0 ? sh.parts : (target + nb - 1) / nb;
+    const long long tiles = (threads + block - 1) / block;
+    long long parts = sh.parts > 0 ? sh.parts
+                                   : adjoint_parts(tiles, nb, (long long)num_sms() * per_sm,
+                                                   t.nC * N * (N + 1), global_gw ? 4.0 : 1e9);
     if (parts > tiles) parts = tiles;
     if (parts < 1) parts = 1;
     plan->block = block;
@@ -264,15 +315,15 @@ static bool plan_td_t(const Tess &t, int nsteps, long long nP, int nb, AdjointPl
     return true;
 }
 
-static bool plan_td_uncached(const Tess &t, int nsteps, int mode, long long nP, int nb,
+static bool plan_td_uncached(const Tess &t, int nsteps, int mode, long long threads, int nb,
                              AdjointPlan *plan, const LaunchShape &sh) {
     const bool small = t.nC <= 256;
 #define CPAB_PLAN(N)                                                                               \
     if (mode != 1)                                                                                 \
-        return small ? plan_td_t<N, 0, uint8_t>(t, nsteps, nP, nb, plan, sh)                       \
-                     : plan_td_t<N, 0, uint16_t>(t, nsteps, nP, nb, plan, sh);                     \
-    return small ? plan_td_t<N, 1, uint8_t>(t, nsteps, nP, nb, plan, sh)                           \
-                 : plan_td_t<N, 1, uint16_t>(t, nsteps, nP, nb, plan, sh);
+        return small ? plan_td_t<N, 0, uint8_t>(t, nsteps, threads, nb, plan, sh)                       \
+                     : plan_td_t<N, 0, uint16_t>(t, nsteps, threads, nb, plan, sh);                     \
+    return small ? plan_td_t<N, 1, uint8_t>(t, nsteps, threads, nb, plan, sh)                           \
+                 : plan_td_t<N, 1, uint16_t>(t, nsteps, threads, nb, plan, sh);
     switch (t.ndim) {
         case 1: { CPAB_PLAN(1) }
         case 2: { CPAB_PLAN(2) }
@@ -281,22 +332,23 @@ static bool plan_td_uncached(const Tess &t, int nsteps, int mode, long long nP, 
 #undef CPAB_PLAN
 }
 
-bool plan_transform_data_backward(const Tess &t, int nsteps, int mode, long long nP, int nb,
+bool plan_transform_data_backward(const Tess &t, int nsteps, int mode, long long threads, int nb,
                                   AdjointPlan *plan, const LaunchShape *force) {
     LaunchShape sh;
-    if (force) return plan_td_uncached(t, nsteps, mode, nP, nb, plan, *force);
-    const bool tuned = tuned_get(kTuneFusedBackward, tune_key(t, nsteps, mode, nP, nb, 0), &sh);
+    if (force) return plan_td_uncached(t, nsteps, mode, threads, nb, plan, *force);
+    const bool tuned = tuned_get(kTuneFusedBackward, tune_key(t, nsteps, mode, threads, nb, 0), &sh);
     // the cache key carries the tuned shape (0: the planner's own)
     const int flag = tuned ? 1 + (sh.staging + 1) + 4 * (sh.block / 32) + 64 * sh.parts : 0;
     static PlanCache cache;
-    return cache.get(1, t, nsteps, mode, nP, nb, flag, plan, [&](AdjointPlan *p) {
-        return plan_td_uncached(t, nsteps, mode, nP, nb, p, sh);
+    return cache.get(1, t, nsteps, mode, threads, nb, flag, plan, [&](AdjointPlan *p) {
+        return plan_td_uncached(t, nsteps, mode, threads, nb, p, sh);
     });
 }
 
 template <int N, int MODE, typename CT>
 static cudaError_t launch_td_bwd_t(const Tess &t, int nsteps, const AdjointPlan &plan,
-                                   const Geo &g, const PreStages &pre, const float *lin,
+                                   const Geo &g, const Patch &patch, const PreStages &pre,
+                                   const float *lin,
                                    const float *table,
                                    const float *grid_saved, int nb, const float *data, int C,
                                    const float *gout, float *ddata, float *partials,
@@ -312,7 +364,7 @@ static cudaError_t launch_td_bwd_t(const Tess &t, int nsteps, const AdjointPlan 
     if (nb > 65535) return cudaErrorInvalidConfiguration;   // images on grid y
     const dim3 grid((unsigned)plan.parts, (unsigned)nb);
     float *gw = plan.gw_floats ? partials + plan.gw_offset() : nullptr;
-    kern<<<grid, plan.block, plan.smem, s>>>(t, nsteps, st, g, pre, lin, table, grid_saved, C,
+    kern<<<grid, plan.block, plan.smem, s>>>(t, nsteps, st, g, patch, pre, lin, table, grid_saved, C,
                                                        data, gout, ddata, partials, gw, plan.parts,
                                                        plan.tiles, ties, err);
     return cudaGetLastError();
@@ -327,29 +379,33 @@ cudaError_t launch_transform_data_backward(const Tess &t, int nsteps, int mode,
                                            unsigned long long *ties, unsigned *err,
                                            cudaStream_t s, const PreStages *pre_in) {
     const Geo g = make_geo(t.ndim, size, outsize);
+    long long threads;
+    const Patch patch = make_patch(t.ndim, outsize, &threads);
+    if ((threads + plan.block - 1) / plan.block != plan.tiles)
+        return cudaErrorInvalidConfiguration;   // not this output's plan
     PreStages pre;
     pre.K = 0;
     if (pre_in) pre = *pre_in;
     const bool small = t.nC <= 256;
 #define CPAB_TDB(N)                                                                             \
     if (mode == 0)                                                                              \
-        return small ? launch_td_bwd_t<N, 0, uint8_t>(t, nsteps, plan, g, pre, lin, table,           \
+        return small ? launch_td_bwd_t<N, 0, uint8_t>(t, nsteps, plan, g, patch, pre, lin, table,           \
                                                       grid_saved, nb, data, C, gout, ddata,     \
                                                       partials, ties, err, s)                   \
-                     : launch_td_bwd_t<N, 0, uint16_t>(t, nsteps, plan, g, pre, lin, table,          \
+                     : launch_td_bwd_t<N, 0, uint16_t>(t, nsteps, plan, g, patch, pre, lin, table,          \
                                                        grid_saved, nb, data, C, gout, ddata,    \
                                                        partials, ties, err, s);                 \
     if (mode == 2)                                                                              \
-        return small ? launch_td_bwd_t<N, 2, uint8_t>(t, nsteps, plan, g, pre, lin, table,           \
+        return small ? launch_td_bwd_t<N, 2, uint8_t>(t, nsteps, plan, g, patch, pre, lin, table,           \
                                                       grid_saved, nb, data, C, gout, ddata,     \
                                                       partials, ties, err, s)                   \
-                     : launch_td_bwd_t<N, 2, uint16_t>(t, nsteps, plan, g, pre, lin, table,          \
+                     : launch_td_bwd_t<N, 2, uint16_t>(t, nsteps, plan, g, patch, pre, lin, table,          \
                                                        grid_saved, nb, data, C, gout, ddata,    \
                                                        partials, ties, err, s);                 \
-    return small ? launch_td_bwd_t<N, 1, uint8_t>(t, nsteps, plan, g, pre, lin, table, grid_saved,   \
+    return small ? launch_td_bwd_t<N, 1, uint8_t>(t, nsteps, plan, g, patch, pre, lin, table, grid_saved,   \
                                                   nb, data, C, gout, ddata, partials, ties,     \
                                                   err, s)                                       \
-                 : launch_td_bwd_t<N, 1, uint16_t>(t, nsteps, plan, g, pre, lin, table, grid_saved,  \
+                 : launch_td_bwd_t<N, 1, uint16_t>(t, nsteps, plan, g, patch, pre, lin, table, grid_saved,  \
                                                    nb, data, C, gout, ddata, partials, ties,    \
                                                    err, s);
     switch (t.ndim) {

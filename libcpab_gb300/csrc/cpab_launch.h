@@ -43,7 +43,7 @@ void tuned_clear();
 // second lookup tier, which only a few warps run, and lose a block (64 x 224^2
 // backward 1.11 against 0.98 ms).  3D keeps its registers.
 template <int N>
-__host__ __device__ constexpr int step_blocks() { return N == 2 ? 4 : 1; }
+__host__ __device__ constexpr int step_blocks() { return N == 1 ? 1 : N == 2 ? 4 : 2; }
 
 // Per-(theta, cell) tables from theta and the basis B [D, d] (fp32):
 // A = B theta, T = expm(dt [A;0]) (rows 0..ndim-1), E = T - I.
@@ -126,7 +126,10 @@ cudaError_t launch_transform_data(const Tess &t, int nsteps, const float *lin, c
                                   unsigned long long *ties, unsigned *err, cudaStream_t s,
                                   const LaunchShape *force = nullptr);
 
-bool plan_transform_data_backward(const Tess &t, int nsteps, int mode, long long nP, int nb,
+// threads: transform_data_backward_threads(ndim, outsize), one per point and
+// a few without one (2D / 3D images are walked in patches).
+long long transform_data_backward_threads(int ndim, const int *outsize);
+bool plan_transform_data_backward(const Tess &t, int nsteps, int mode, long long threads, int nb,
                                   AdjointPlan *plan, const LaunchShape *force = nullptr);
 
 // Transformations applied to the grid before the one being differentiated

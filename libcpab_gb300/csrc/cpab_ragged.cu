@@ -199,9 +199,11 @@ __host__ __device__ inline size_t ragged_adjoint_smem(int nC, int nsteps, int bl
 struct LaneSlotSink {
     float *ls;
     int lo, hi;
+    static constexpr bool kWarp = false;   // changed() is called by the leaving lanes alone
     template <int P>
-    __device__ __forceinline__ void operator()(bool flush, int cell, const float (&acc)[P]) {
-        if (flush) {
+    __device__ __forceinline__ void changed(unsigned, bool change, int cell,
+                                            const float (&acc)[P]) {
+        if (change) {
             float *q = ls + cell * (P * 32) + (threadIdx.x & 31);
 #pragma unroll
             for (int i = 0; i < P; ++i) atomicAdd(q + i * 32, acc[i]);
@@ -338,8 +340,8 @@ __global__ void __launch_bounds__(256)
                               gf);
                 lam[0] = gf[0] * g.sizem1[0];
             }
-            if constexpr (LS) reverse_sweep_to<1, MODE, CT>(sm, nsteps, st, live, lam, slots);
-            else reverse_sweep<1, MODE, CT>(sm, nsteps, st, live, lam, sm.gw);
+            if constexpr (LS) reverse_sweep_to<1, MODE, CT>(sm, nsteps, st, lam, slots);
+            else reverse_sweep<1, MODE, CT, false, true>(sm, nsteps, st, lam, sm.gw);
         }
     }
     finish(s);

@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256, 3)
                 lam[r] = live ? __ldg(gout + r * total + base + j) : 0.f;
             }
             logged_forward<N, MODE, CT>(sm, t, nsteps, st, p, ties, err);
-            reverse_sweep<N, MODE, CT>(sm, nsteps, st, live, lam, sm.gw);
+            reverse_sweep<N, MODE, CT, false, true>(sm, nsteps, st, lam, sm.gw);
             if (dpoints && live) {
 #pragma unroll
                 for (int r = 0; r < N; ++r) dpoints[r * total + base + j] = lam[r];
