@@ -48,6 +48,31 @@ def _basis(params, device):
     return basis_on(params, device)
 
 
+def settings(params, device):
+    """What a forward or backward reads from params when it runs: (nsteps,
+    mode, point_gradient, tie counter or None, basis on the device)."""
+    return (int(params.nstepsolver), _mode(params), bool(getattr(params, 'point_gradient', False)),
+            _ties(params), _basis(params, device))
+
+
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+_functorch_level = torch._C._functorch.peek_interpreter_stack
+_function_modes = torch._C._len_torch_function_stack
+_dispatch_modes = torch._C._len_torch_dispatch_stack
+
+
+def native(*tensors):
+    """Whether the native nodes (csrc/torch_bind.cpp) may take a call: plain
+    tensors, and nobody watching the Python autograd functions (functorch
+    transforms, forward-mode AD, tracing, function or dispatch modes)."""
+    for t in tensors:
+        if type(t) not in _PLAIN:
+            return False
+    return (_functorch_level() is None and _function_modes() == 0 and _dispatch_modes() == 0
+            and torch.autograd.forward_ad._current_level < 0
+            and torch._C._get_tracing_state() is None)
+
+
 class TransformGrid(torch.autograd.Function):
     @staticmethod
     def forward(ctx, points, theta, params):

@@ -126,6 +126,28 @@ def load(path: str | None = None):
         return lib
 
 
+_bind = None
+
+
+def bind():
+    """The torch extension _torch_bind (native autograd nodes), loaded once."""
+    global _bind
+    if _bind is None:
+        load()   # its own message if the C ABI library is missing
+        with _lock:
+            if _bind is None:
+                path = os.path.join(HERE, '_torch_bind.so')
+                if not os.path.exists(path):
+                    raise ImportError('libcpab_gb300 torch extension not found at %s; build it '
+                                      'with "python -m libcpab_gb300.build"' % path)
+                import importlib.util
+                spec = importlib.util.spec_from_file_location('libcpab_gb300._torch_bind', path)
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+                _bind = mod
+    return _bind
+
+
 def _check(rc: int):
     if rc != 0:
         msg = load().cpab_last_error().decode(errors='replace')

@@ -1,4 +1,5 @@
-"""Build the sm_103a shared library libcpab_gb300/libcpab_gb300.so.
+"""Build the sm_103a shared library libcpab_gb300/libcpab_gb300.so and the
+torch extension libcpab_gb300/_torch_bind.so over it.
 
 Each translation unit in csrc/ is compiled by nvcc in parallel
 (-gencode arch=compute_103a,code=sm_103a) and linked into one shared library
@@ -18,6 +19,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, 'csrc')
 BUILD = os.path.join(HERE, '_build')
 LIB = os.path.join(HERE, 'libcpab_gb300.so')
+BIND = os.path.join(HERE, '_torch_bind.so')
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 
 
@@ -40,20 +42,55 @@ def _compile(nvcc, src, obj, verbose):
     return r.stderr
 
 
+def _compile_bind(src, obj):
+    """The native autograd nodes, against the installed torch (host code only)."""
+    import sysconfig
+    import torch
+    root = os.path.join(os.path.dirname(torch.__file__), 'include')
+    cuda = os.path.dirname(os.path.dirname(nvcc_path()))
+    cmd = ['g++', '-O2', '-std=c++17', '-fPIC', '-fvisibility=hidden',
+           '-D_GLIBCXX_USE_CXX11_ABI=%d' % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+    for d in (root, os.path.join(root, 'torch', 'csrc', 'api', 'include'),
+              sysconfig.get_paths()['include'], os.path.join(cuda, 'include')):
+        cmd += ['-isystem', d]
+    r = subprocess.run(cmd + ['-c', src, '-o', obj], capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError('g++ failed for %s:\n%s' % (src, r.stderr))
+
+
+def _link_bind(obj):
+    import torch
+    lib = os.path.join(os.path.dirname(torch.__file__), 'lib')
+    tmp = BIND + '.tmp%d' % os.getpid()
+    # the C ABI library sits next to the extension and is found through $ORIGIN
+    cmd = ['g++', '-shared', '-o', tmp, obj, '-L' + HERE, '-l:libcpab_gb300.so', '-L' + lib,
+           '-ltorch_python', '-ltorch', '-ltorch_cpu', '-lc10', '-lc10_cuda',
+           '-Wl,-rpath,$ORIGIN']
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError('link failed:\n' + r.stderr)
+    os.replace(tmp, BIND)
+
+
 def build(force=False, verbose=False):
-    """Compile if any source is newer than the library; returns the .so path."""
+    """Compile if any source is newer than the libraries; returns the .so path
+    of the C ABI."""
     srcs = sorted(glob.glob(os.path.join(CSRC, '*.cu')))
+    bind_src = os.path.join(CSRC, 'torch_bind.cpp')
     deps = srcs + glob.glob(os.path.join(CSRC, '*.cuh')) + glob.glob(os.path.join(CSRC, '*.h')) + \
-        [os.path.join(os.path.dirname(HERE), 'include', 'cpab_gb300.h'), __file__]
-    if not force and os.path.exists(LIB):
-        t = os.path.getmtime(LIB)
+        [bind_src, os.path.join(os.path.dirname(HERE), 'include', 'cpab_gb300.h'), __file__]
+    if not force and os.path.exists(LIB) and os.path.exists(BIND):
+        t = min(os.path.getmtime(LIB), os.path.getmtime(BIND))
         if all(os.path.getmtime(d) <= t for d in deps if os.path.exists(d)):
             return LIB
     os.makedirs(BUILD, exist_ok=True)
     nvcc = nvcc_path()
     objs = [os.path.join(BUILD, os.path.basename(s)[:-3] + '.o') for s in srcs]
-    with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    bind_obj = os.path.join(BUILD, 'torch_bind.o')
+    with concurrent.futures.ThreadPoolExecutor(max_workers=min(9, len(srcs) + 1)) as ex:
+        bind = ex.submit(_compile_bind, bind_src, bind_obj)
         logs = list(ex.map(lambda so: _compile(nvcc, so[0], so[1], verbose), zip(srcs, objs)))
+        bind.result()
     if verbose:
         for s, lg in zip(srcs, logs):
             print('==', os.path.basename(s))
@@ -64,6 +101,7 @@ def build(force=False, verbose=False):
     if r.returncode != 0:
         raise RuntimeError('link failed:\n' + r.stderr)
     os.replace(tmp, LIB)
+    _link_bind(bind_obj)
     return LIB
 
 

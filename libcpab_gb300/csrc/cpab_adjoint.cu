@@ -179,8 +179,7 @@ static cudaError_t launch_adjoint_t(const Tess &t, int nsteps, const AdjointPlan
     auto kern = k_adjoint<N, MODE, CT, false>;
     if constexpr (N >= 2)
         if (plan.gw_floats) kern = k_adjoint<N, MODE, CT, true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)plan.smem);
+    cudaError_t e = allow_smem((const void *)kern, plan.smem);
     if (e != cudaSuccess) return e;
     const Steps st = make_steps(nsteps);
     if (n_theta == 0) return cudaSuccess;

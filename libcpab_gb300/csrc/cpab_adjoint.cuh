@@ -228,11 +228,8 @@ inline bool adjoint_shape(K kern_shared, K kern_global, int nC, int nsteps, int 
             const size_t sm = adjoint_smem_bytes<N, CT>(nC, nsteps, b, g == 0) + 64;
             if (sm > (size_t)max_optin) continue;
             const K kern = g == 0 ? kern_shared : kern_global;
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sm) != cudaSuccess)
-                return false;
-            int n = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, b, sm);
+            if (allow_smem((const void *)kern, sm) != cudaSuccess) return false;
+            const int n = resident_blocks((const void *)kern, b, sm);
             if (n * (b / 32) > best) {
                 best = n * (b / 32);
                 *block = b;

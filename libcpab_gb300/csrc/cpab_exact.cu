@@ -208,11 +208,7 @@ cudaError_t launch_integrate_exact(const Tess &t, const float *points, int broad
 #define CPAB_EX(N)                                                                            \
     {                                                                                         \
         auto kern = k_integrate_exact<N>;                                                     \
-        if (smem > 48 * 1024) {                                                               \
-            cudaError_t e = cudaFuncSetAttribute(                                             \
-                kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                \
-            if (e != cudaSuccess) return e;                                                   \
-        }                                                                                     \
+        if (const cudaError_t e = allow_smem((const void *)kern, smem)) return e;            \
         kern<<<grid, block, smem, s>>>(t, points, broadcast, nP, A, (int)tiles, out, ties, err, \
                                        iters);                                                \
         return cudaGetLastError();                                                            \
@@ -494,9 +490,7 @@ cudaError_t launch_adjoint_exact(const Tess &t, const AdjointPlan &plan, const f
 #define CPAB_AEX(N)                                                                           \
     {                                                                                         \
         auto kern = k_adjoint_exact<N>;                                                       \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                             (int)plan.smem);                                 \
-        if (e != cudaSuccess) return e;                                                       \
+        if (const cudaError_t e = allow_smem((const void *)kern, plan.smem)) return e;         \
         kern<<<grid, plan.block, plan.smem, s>>>(t, out, nP, A, plan.parts, plan.tiles, gout, \
                                                  dpoints, partials, ties, err);               \
         return cudaGetLastError();                                                            \

@@ -231,11 +231,7 @@ static cudaError_t launch_finalize_t(int nC, const Steps &st, const Partials &ps
         K *= 2;
     const size_t smem = bytes(K);
     auto kern = k_finalize<N, MODE>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    if (const cudaError_t e = allow_smem((const void *)kern, smem)) return e;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = K;

@@ -207,11 +207,7 @@ cudaError_t launch_transform_data(const Tess &t, int nsteps, const float *lin, c
 #define CPAB_TD(N, PP)                                                                         \
     {                                                                                          \
         auto kern = k_transform_data<N, PP>;                                                   \
-        if (smem > 48 * 1024) {                                                                \
-            cudaError_t e = cudaFuncSetAttribute(                                              \
-                kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                 \
-            if (e != cudaSuccess) return e;                                                    \
-        }                                                                                      \
+        if (const cudaError_t e = allow_smem((const void *)kern, smem)) return e;            \
         kern<<<grid, block, smem, s>>>(t, nsteps, g, lin, E, C, data, out, grid_out, \
                                                  tiles, ties, err);                            \
         return cudaGetLastError();                                                             \
@@ -356,8 +352,7 @@ static cudaError_t launch_td_bwd_t(const Tess &t, int nsteps, const AdjointPlan 
     auto kern = k_transform_data_backward<N, MODE, CT, false>;
     if constexpr (N >= 2)
         if (plan.gw_floats) kern = k_transform_data_backward<N, MODE, CT, true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)plan.smem);
+    cudaError_t e = allow_smem((const void *)kern, plan.smem);
     if (e != cudaSuccess) return e;
     const Steps st = make_steps(nsteps);
     if (nb == 0) return cudaSuccess;

@@ -17,6 +17,7 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <tuple>
 
 #include "cpab_launch.h"
 
@@ -82,11 +83,7 @@ static cudaError_t launch_integrate_t(const Tess &t, int nsteps, const float *po
     const dim3 grid((unsigned)tiles, (unsigned)n_theta);
     const size_t smem = (size_t)t.nC * N * (N + 1) * sizeof(float);
     auto kern = k_integrate<N, COMP, PPT>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    if (const cudaError_t e = allow_smem((const void *)kern, smem)) return e;
     kern<<<grid, block, smem, s>>>(t, nsteps, points, broadcast, nP, table, tiles, out,
                                              trace, ties, err);
     return cudaGetLastError();
@@ -194,6 +191,45 @@ void tuned_set(int kind, const TuneKey &key, const LaunchShape &shape) {
 void tuned_clear() {
     std::lock_guard<std::mutex> lock(g_shape_mu);
     g_shapes.clear();
+}
+
+static int current_device() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        dev = 0;
+    }
+    return dev;
+}
+
+cudaError_t allow_smem(const void *kernel, size_t bytes) {
+    if (bytes <= 46 * 1024) return cudaSuccess;   // 48 KB with the static shared memory
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> allowed;   // one entry per kernel
+    const auto key = std::make_pair(current_device(), kernel);
+    std::lock_guard<std::mutex> lock(mu);
+    size_t &most = allowed[key];
+    if (bytes <= most) return cudaSuccess;
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) most = bytes;
+    return e;
+}
+
+int resident_blocks(const void *kernel, int block, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, const void *, int, size_t>, int> known;
+    const auto key = std::make_tuple(current_device(), kernel, block, smem);
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (known.size() > 4096) known.clear();
+    return known[key] = n;
 }
 
 // SM count of the current device, looked up once per device (relaxed atomics:

@@ -45,6 +45,13 @@ void tuned_clear();
 template <int N>
 __host__ __device__ constexpr int step_blocks() { return N == 1 ? 1 : N == 2 ? 4 : 2; }
 
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) where a launch needs it (near
+// or above 48 KB), once per kernel, device and size; and the occupancy query, kept
+// per kernel, device, block and size.  Both cost microseconds of host time, on
+// every launch of an eager step.
+cudaError_t allow_smem(const void *kernel, size_t bytes);
+int resident_blocks(const void *kernel, int block, size_t smem);   // 0: does not fit
+
 // Per-(theta, cell) tables from theta and the basis B [D, d] (fp32):
 // A = B theta, T = expm(dt [A;0]) (rows 0..ndim-1), E = T - I.
 cudaError_t launch_cell_tables(const Tess &t, int nsteps, const float *theta, int n_theta, int d,

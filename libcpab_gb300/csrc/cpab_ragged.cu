@@ -414,13 +414,8 @@ static cudaError_t launch_rf_t(const Tess &t, int nsteps, int block, int S, cons
                                cudaStream_t s) {
     auto kern = k_ragged_forward<PPT>;
     const size_t smem = (size_t)(block / 32) * round4(t.nC * 2) * 4;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem);
+    if (const cudaError_t e = allow_smem((const void *)kern, smem)) return e;
+    const int per_sm = resident_blocks((const void *)kern, block, smem);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     kern<<<num_sms() * per_sm, block, smem, s>>>(t, nsteps, S, off, tile_off, E, values, out,
                                                   ties, err);
@@ -452,11 +447,9 @@ static cudaError_t launch_ra_ls(const Tess &t, int nsteps, int block, int ppt, i
                                 unsigned long long *ties, unsigned *err, cudaStream_t s) {
     auto kern = k_ragged_adjoint<MODE, CT, FUSED, LS>;
     const size_t smem = ragged_adjoint_smem<MODE, CT>(t.nC, nsteps, block);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem);
+    const int per_sm = resident_blocks((const void *)kern, block, smem);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     // partial slots are sized for at most 64 resident warps per SM, lane slots
     // for kLaneSlotWarpsPerSM

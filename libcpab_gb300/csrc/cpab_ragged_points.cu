@@ -203,13 +203,8 @@ static cudaError_t launch_rpf_t(const Tess &t, int nsteps, int S, const long lon
                                 unsigned *err, cudaStream_t s, int block) {
     auto kern = k_ragged_points_forward<N, PPT>;
     const size_t smem = (size_t)(block / 32) * round4(t.nC * N * (N + 1)) * 4;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem);
+    if (const cudaError_t e = allow_smem((const void *)kern, smem)) return e;
+    const int per_sm = resident_blocks((const void *)kern, block, smem);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     kern<<<num_sms() * per_sm, block, smem, s>>>(t, nsteps, S, off, tile_off, E, total, points,
                                                   out, ties, err);
@@ -284,11 +279,9 @@ static cudaError_t launch_rpa_t(const Tess &t, int nsteps, int S, const long lon
     if (!block) return cudaErrorInvalidConfiguration;
     auto kern = k_ragged_points_adjoint<N, MODE, CT>;
     const size_t smem = points_adjoint_smem<N, CT>(t.nC, nsteps, block);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem);
+    const int per_sm = resident_blocks((const void *)kern, block, smem);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     const int W = block / 32;
     // partial slots are sized for at most 64 resident warps per SM

@@ -113,11 +113,7 @@ cudaError_t launch_sequential_transform_data(const SeqStages &sq, const float *l
 #define CPAB_SQ(N, PP)                                                                        \
     {                                                                                         \
         auto kern = k_sequential_transform_data<N, PP>;                                       \
-        if (smem > 48 * 1024) {                                                               \
-            cudaError_t e = cudaFuncSetAttribute(                                             \
-                kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                \
-            if (e != cudaSuccess) return e;                                                   \
-        }                                                                                     \
+        if (const cudaError_t e = allow_smem((const void *)kern, smem)) return e;            \
         kern<<<grid, block, smem, s>>>(sq, g, lin, C, data, out, grid_out, ties, err);        \
         return cudaGetLastError();                                                            \
     }
