@@ -143,33 +143,19 @@ __device__ __forceinline__ CornerStep<N> corner_steps(const float (&p)[N], const
 // bit 0), and so on.
 
 // d(lerp)/d(f_j) and the per-corner weights, for the backward passes.
-// Where the clamp puts both corners of an axis on one element (points beyond
-// the edge), that element gets the whole weight in one addition: the two parts
-// (1 - f) w and f w cancel to w, and added to memory one after the other they
-// left the rounding of |f| w there (|f| reaches thousands for points far out).
-// A weight that is not finite stays so.
 template <int N>
 __device__ __forceinline__ void lerp_grads(const float *D, const Corner<N> &cr, float w,
                                            float *ddata_plane, float (&gf)[N]) {
     float v[1 << N];
 #pragma unroll
     for (int m = 0; m < (1 << N); ++m) v[m] = __ldg(D + cr.off[m]);
-    if (ddata_plane) {
-        float lo[N], hi[N];
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
-            const bool one = cr.off[1 << j] == cr.off[0];
-            lo[j] = one ? fmaf(0.f, cr.f[j], 1.f) : 1.f - cr.f[j];
-            hi[j] = one ? 0.f : cr.f[j];
-        }
+    for (int m = 0; m < (1 << N); ++m) {
+        // chain order of autograd: last lerp (highest axis) first
+        float wt = w;
 #pragma unroll
-        for (int m = 0; m < (1 << N); ++m) {
-            // chain order of autograd: last lerp (highest axis) first
-            float wt = w;
-#pragma unroll
-            for (int j = N - 1; j >= 0; --j) wt *= ((m >> j) & 1) ? hi[j] : lo[j];
-            if (wt != 0.f) atomicAdd(ddata_plane + cr.off[m], wt);
-        }
+        for (int j = N - 1; j >= 0; --j) wt *= ((m >> j) & 1) ? cr.f[j] : (1.f - cr.f[j]);
+        if (ddata_plane) atomicAdd(ddata_plane + cr.off[m], wt);
     }
 #pragma unroll
     for (int j = 0; j < N; ++j) {
