@@ -711,19 +711,22 @@ struct PointOrder {
 constexpr int kMaxRow = 1024;   // rows looked for (four reads of a 256-thread block)
 
 // Called by all threads of the block; `found` is shared.
-template <int N>
+// MOVED: the points are a meshgrid that a transformation has moved; its rows are
+// told by the jump back of the first coordinate instead.
+template <int N, bool MOVED = false>
 __device__ __forceinline__ PointOrder point_order(const float *points, long long nP, int *found) {
     PointOrder o = {0, 32, 5};
     if constexpr (N >= 2) {
         if (nP < 64 || nP >= (1ll << 31)) return o;
         if (threadIdx.x == 0) *found = kMaxRow + 1;
         __syncthreads();
-        const float *y = points + nP;
+        const float *y = points + (MOVED ? 0 : nP);
         const float y0 = __ldg(y);
         const int most = (int)min(nP, (long long)kMaxRow + 1);
         int row = kMaxRow + 1;
         for (int i = 1 + threadIdx.x; i - (int)threadIdx.x < most; i += blockDim.x) {
-            if (i < most && __ldg(y + i) != y0) atomicMin(found, i);
+            if (i < most && (MOVED ? __ldg(y + i) < __ldg(y + i - 1) - 0.25f : __ldg(y + i) != y0))
+                atomicMin(found, i);
             __syncthreads();
             row = *found;
             __syncthreads();

@@ -18,14 +18,13 @@
 //     edge cells extend past it), the speed within distance d + e of p is at
 //     most |v(p)| + ||A_lin|| (d + e), so a step of time (d + e) / that bound
 //     stays in the cell or passes a face by at most e = 1e-5 (where the two
-//     cells' fields differ by O(e)).  Each step uses the exact in-cell flow
-//     E(dt); the cell is looked up with the reference's rules before each
-//     step.  Steps shrink geometrically towards a face, so a crossing costs
+//     cells' fields differ by O(e)).  Each step uses the exact in-cell flow,
+//     p + sum_k dt^k A_lin^(k-1) v / k! (|A| dt < 1 by the rule; the series on
+//     the vector takes 60 operations where the matrix E(dt) took 180); the cell
+//     is looked up with the reference's rules before each step.  Steps shrink geometrically towards a face, so a crossing costs
 //     ~10-20 steps; a trajectory that needs more than kExactMaxIter steps
 //     raises kErrIterLimit and returns its position at that point.
 #include "cpab_adjoint.cuh"
-#include "cpab_expm.cuh"
-#include "cpab_frechet.cuh"
 
 namespace cpab {
 
@@ -123,6 +122,70 @@ __device__ __forceinline__ float face_distance(const float (&p)[N], const Tess &
     return fmaxf(d - 4e-7f * imin, 0.f);
 }
 
+// Square root to 1-2 ulp in one instruction (the step bounds carry more slack
+// than that; the rounded one and the rounded division were a fifth of the
+// dependent chain of a step, and a trajectory that slides along a face takes
+// thousands of steps one after the other).
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Velocity at p in cell map M, and the certified step there; negative for a
+// field that vanishes at p and has no linear part, or NaN input.
+template <int N>
+__device__ __forceinline__ float certified_step(const float (&M)[N * (N + 1)], const float (&p)[N],
+                                                float (&v)[N], float &norm, const Tess &t) {
+    float speed2 = 0.f, anorm2 = 0.f;
+    affine_apply<N>(M, p, v);
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        speed2 = fmaf(v[r], v[r], speed2);
+#pragma unroll
+        for (int k = 0; k < N; ++k) anorm2 = fmaf(M[r * (N + 1) + k], M[r * (N + 1) + k], anorm2);
+    }
+    const float reach = face_distance<N>(p, t) + kOvershoot;
+    norm = sqrt_approx(anorm2);
+    const float bound = sqrt_approx(speed2) + norm * reach;
+    return bound > 0.f ? __fdividef(reach, bound) : -1.f;
+}
+
+// Terms of the in-cell flow's series: with |A| dt < 1 the first one left out is
+// below 1 / 12! = 2e-9 of the step; below kShortStep (steps shrink towards a
+// face), kShortTerms leave less than that.  Each lane decides for itself, so its
+// result does not depend on its neighbours.
+constexpr int kFlowTerms = 11, kShortTerms = 5;
+constexpr float kShortStep = 0.06f;
+
+// p + sum_{k=1..K} term_k, term_1 = dt v, term_{k+1} = dt A_lin term_k / (k + 1)
+template <int N, int K>
+__device__ __forceinline__ void flow_step(const float (&M)[N * (N + 1)], const float (&v)[N],
+                                          float dt, float (&p)[N]) {
+    float term[N], sum[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) sum[r] = term[r] = dt * v[r];
+#pragma unroll
+    for (int k = 2; k <= K; ++k) {
+        float nt[N];
+        const float f = dt * (1.f / (float)k);
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            float q = 0.f;
+#pragma unroll
+            for (int j = 0; j < N; ++j) q = fmaf(M[r * (N + 1) + j], term[j], q);
+            nt[r] = f * q;
+        }
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            term[r] = nt[r];
+            sum[r] += nt[r];
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < N; ++r) p[r] += sum[r];
+}
+
 template <int N>
 __device__ void exact_flow_nd(float (&p)[N], const float *tab, const Tess &t,
                               unsigned long long *ties, unsigned *err,
@@ -132,38 +195,13 @@ __device__ void exact_flow_nd(float (&p)[N], const float *tab, const Tess &t,
     int it = 0;
     for (; it < kExactMaxIter && tr > 0.f; ++it) {
         const int c = find_cell<N>(p, t, ties);
-        float M[P];
+        float M[P], v[N], norm;
         load_cell<N>(tab, c, M);
-        float v[N], speed2 = 0.f, anorm2 = 0.f;
-        affine_apply<N>(M, p, v);
-#pragma unroll
-        for (int r = 0; r < N; ++r) {
-            speed2 = fmaf(v[r], v[r], speed2);
-#pragma unroll
-            for (int k = 0; k < N; ++k) anorm2 = fmaf(M[r * (N + 1) + k], M[r * (N + 1) + k], anorm2);
-        }
-        const float reach = face_distance<N>(p, t) + kOvershoot;
-        const float bound = sqrtf(speed2) + sqrtf(anorm2) * reach;
-        if (!(bound > 0.f)) break;                   // at rest (or non-finite)
-        const float dt = fminf(tr, reach / bound);
-        float Ml[N][N], vt[N], El[N][N], Et[N];
-#pragma unroll
-        for (int r = 0; r < N; ++r) {
-#pragma unroll
-            for (int k = 0; k < N; ++k) Ml[r][k] = dt * M[r * (N + 1) + k];
-            vt[r] = dt * M[r * (N + 1) + N];
-        }
-        expm1_affine<N>(Ml, vt, El, Et);
-        float q[N];
-#pragma unroll
-        for (int r = 0; r < N; ++r) {
-            float acc = Et[r];
-#pragma unroll
-            for (int k = 0; k < N; ++k) acc = fmaf(El[r][k], p[k], acc);
-            q[r] = p[r] + acc;
-        }
-#pragma unroll
-        for (int r = 0; r < N; ++r) p[r] = q[r];
+        const float step = certified_step<N>(M, p, v, norm, t);
+        if (step < 0.f) break;                       // at rest (or non-finite)
+        const float dt = fminf(tr, step);
+        if (norm * dt < kShortStep) flow_step<N, kShortTerms>(M, v, dt, p);
+        else flow_step<N, kFlowTerms>(M, v, dt, p);
         tr -= dt;
     }
     if (it >= kExactMaxIter) raise_error(err, kErrIterLimit);
@@ -179,13 +217,17 @@ __global__ void __launch_bounds__(256)
     constexpr int P = N * (N + 1);
     extern __shared__ float4 smem4[];
     __shared__ uint64_t bar;
+    __shared__ int found;
     float *tab = reinterpret_cast<float *>(smem4);
     const int th = blockIdx.y;
     const int G = t.nC * P;
-    if (!stage_table(tab, A + (long long)th * G, G, &bar, err)) return;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= nP) return;
     const float *src = points + (broadcast ? (long long)th * N * nP : 0ll);
+    // neighbours cross faces at about the same time: patches even out the steps
+    const PointOrder order = point_order<N>(src, nP, &found);
+    if (!stage_table(tab, A + (long long)th * G, G, &bar, err)) return;
+    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nP) return;
+    const long long idx = ordered_point(v, order);
     float p[N];
 #pragma unroll
     for (int r = 0; r < N; ++r) p[r] = __ldg(src + r * nP + idx);
@@ -234,15 +276,110 @@ cudaError_t launch_integrate_exact(const Tess &t, const float *points, int broad
 // of p and steps back, p_prev = expm(-dt X_c) p~ (X_c = [A_c; 0]).  For that
 // sub-step, read forwards as q' = T q with T = expm(dt X_c):
 //     lambda_prev = T_lin^T lambda,
-//     dL/dA_c += dt [L_exp(dt X_c^T, [lambda p~_prev^T; 0])]_{top rows}
-// (the adjoint Frechet derivative of expm, as in the exact mode of the
-// fixed-step adjoint).  A sub-step that passed a face (by at most 1e-5, as in
+//     dL/dA_c += integral of lambda(t) p~(t)^T over the sub-step,
+// lambda(t) and p(t) the cotangent and the point on the way, from their series:
+// Gauss-Legendre quadrature (back_step).  (The adjoint Frechet derivative of
+// expm, used before, is the same integral at four times the operations.)  A
+// sub-step that passed a face (by at most 1e-5, as in
 // the forward) is corrected to first order in the time it spent on the far
 // side, so the overshoot costs the derivative only at second order.
 // dL/dA_c accumulates per lane while the lane stays in
 // a cell and is flushed into the warp's cell table with warp_flush (fixed
 // summation order: dtheta is reproducible).  The loop runs until every lane
 // of the warp has used up its time, so all lanes reach every flush.
+// Gauss-Legendre nodes and weights on [0, 1].
+template <int G>
+__device__ __forceinline__ constexpr float gauss_node(int n) {
+    if (G == 2) return n == 0 ? 0.21132486540518711775f : 0.78867513459481288225f;
+    return n == 0   ? 0.06943184420297371239f
+           : n == 1 ? 0.33000947820757186760f
+           : n == 2 ? 0.66999052179242813240f
+                    : 0.93056815579702628761f;
+}
+template <int G>
+__device__ __forceinline__ constexpr float gauss_weight(int n) {
+    if (G == 2) return 0.5f;
+    return n == 0 || n == 3 ? 0.17392742256872692869f : 0.32607257743127307131f;
+}
+
+// One sub-step back over dt from p (velocity v of the forward field M) with the
+// cotangent lam: q [p_prev; 1], nl = lambda_prev, and acc += the integral of
+// lambda [p; 1]^T.  K terms of the series of both at G nodes and at the end: for
+// |A| dt < 1, 11 terms and 4 nodes (error below 6e-10 (2 |A| dt)^8 <= 1.5e-7 of
+// the integrand), below kShortStep 5 and 2 ((2 |A| dt)^4 / 4320 <= 5e-8).
+template <int N, int K, int G>
+__device__ __forceinline__ void back_step(const float (&M)[N * (N + 1)], const float (&p)[N],
+                                          const float (&v)[N], const float (&lam)[N], float dt,
+                                          float (&acc)[N * (N + 1)], float (&q)[N + 1],
+                                          float (&nl)[N]) {
+    float tp[N], tl[N], sp[G + 1][N], sl[G + 1][N], power[G];
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        tp[r] = -dt * v[r];
+        tl[r] = lam[r];
+        sp[G][r] = tp[r];
+        sl[G][r] = lam[r];
+    }
+#pragma unroll
+    for (int n = 0; n < G; ++n) {
+        power[n] = gauss_node<G>(n);
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            sp[n][r] = power[n] * tp[r];
+            sl[n][r] = lam[r];
+        }
+    }
+#pragma unroll
+    for (int k = 1; k <= K; ++k) {
+        const float fl = dt * (1.f / (float)k), fp = -dt * (1.f / (float)(k + 1));
+        float np[N], nt[N];
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            float a = 0.f, b = 0.f;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                a = fmaf(M[r * (N + 1) + j], tp[j], a);
+                b = fmaf(M[j * (N + 1) + r], tl[j], b);
+            }
+            np[r] = fp * a;
+            nt[r] = fl * b;
+        }
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            tp[r] = np[r];
+            tl[r] = nt[r];
+            sl[G][r] += tl[r];
+            sp[G][r] += tp[r];
+        }
+#pragma unroll
+        for (int n = 0; n < G; ++n) {   // node^k for the cotangent, node^(k+1) for the point
+#pragma unroll
+            for (int r = 0; r < N; ++r) sl[n][r] = fmaf(power[n], tl[r], sl[n][r]);
+            power[n] *= gauss_node<G>(n);
+#pragma unroll
+            for (int r = 0; r < N; ++r) sp[n][r] = fmaf(power[n], tp[r], sp[n][r]);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < G; ++n) {
+        const float w = gauss_weight<G>(n) * dt;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float l = w * sl[n][i];
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+                acc[i * (N + 1) + j] = fmaf(l, p[j] + sp[n][j], acc[i * (N + 1) + j]);
+            acc[i * (N + 1) + N] += l;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        q[r] = p[r] + sp[G][r];
+        nl[r] = sl[G][r];
+    }
+    q[N] = 1.f;
+}
+
 template <int N>
 __global__ void __launch_bounds__(128)
     k_adjoint_exact(const __grid_constant__ Tess t, const float *__restrict__ out, long long nP,
@@ -252,18 +389,20 @@ __global__ void __launch_bounds__(128)
     constexpr int P = N * (N + 1);
     extern __shared__ float4 smem4[];
     __shared__ uint64_t bar;
+    __shared__ int found;
     const int B = blockDim.x, W = B / 32, tid = threadIdx.x;
     const int th = blockIdx.y, part = blockIdx.x;
     const int G = t.nC * P, Gr = round4(G);
     float *tab = reinterpret_cast<float *>(smem4);
     float *gw = tab + Gr;
+    const PointOrder order = point_order<N, true>(out + (long long)th * N * nP, nP, &found);
     if (!stage_table(tab, A + (long long)th * G, G, &bar, err)) return;
     for (int i = tid; i < W * Gr; i += B) gw[i] = 0.f;
     __syncthreads();
     float *warp_tab = gw + (size_t)(tid >> 5) * Gr;
     for (int tile = part; tile < tiles; tile += parts) {
-        const long long idx = (long long)tile * B + tid;
-        const bool live = idx < nP;
+        const bool live = (long long)tile * B + tid < nP;
+        const long long idx = ordered_point((long long)tile * B + tid, order);
         float p[N], lam[N], acc[P];
 #pragma unroll
         for (int r = 0; r < N; ++r) {
@@ -283,24 +422,14 @@ __global__ void __launch_bounds__(128)
         for (int i = 0; i < P; ++i) pend[i] = 0.f;
         while (__any_sync(0xffffffffu, tr > 0.f)) {
             const bool act = tr > 0.f;
-            float M[P];
+            float M[P], v[N], norm = 0.f;
             float dt = 0.f;
             if (act) {
                 load_cell<N>(tab, cc, M);
-                float v[N], speed2 = 0.f, anorm2 = 0.f;
-                affine_apply<N>(M, p, v);
-#pragma unroll
-                for (int r = 0; r < N; ++r) {
-                    speed2 = fmaf(v[r], v[r], speed2);
-#pragma unroll
-                    for (int k = 0; k < N; ++k)
-                        anorm2 = fmaf(M[r * (N + 1) + k], M[r * (N + 1) + k], anorm2);
-                }
-                const float reach = face_distance<N>(p, t) + kOvershoot;
-                const float bound = sqrtf(speed2) + sqrtf(anorm2) * reach;
+                const float step = certified_step<N>(M, p, v, norm, t);
                 // a cell whose field vanishes at p and has no linear part is
                 // at rest everywhere: the remaining time in one sub-step
-                dt = (bound > 0.f) ? fminf(tr, reach / bound) : tr;
+                dt = (step >= 0.f) ? fminf(tr, step) : tr;
                 if (!(dt > 0.f)) dt = tr;   // non-finite input: stop below
             }
             const bool change = act && cc != gcell;
@@ -314,48 +443,12 @@ __global__ void __launch_bounds__(128)
                 }
             }
             if (act) {
-                // the sub-step's start: q = p + (expm(-dt X) - I) p~
-                float Ml[N][N], vt[N], El[N][N], Et[N];
-#pragma unroll
-                for (int r = 0; r < N; ++r) {
-#pragma unroll
-                    for (int k = 0; k < N; ++k) Ml[r][k] = -dt * M[r * (N + 1) + k];
-                    vt[r] = -dt * M[r * (N + 1) + N];
-                }
-                expm1_affine<N>(Ml, vt, El, Et);
-                float q[N + 1];
-#pragma unroll
-                for (int r = 0; r < N; ++r) {
-                    float a = Et[r];
-#pragma unroll
-                    for (int k = 0; k < N; ++k) a = fmaf(El[r][k], p[k], a);
-                    q[r] = p[r] + a;
-                }
-                q[N] = 1.f;
-                // Y = dt X^T; direction [lambda q^T; 0]
-                float Y[N + 1][N + 1], Wd[N + 1][N + 1], L[N + 1][N + 1], R[N + 1][N + 1];
-#pragma unroll
-                for (int i = 0; i <= N; ++i)
-#pragma unroll
-                    for (int j = 0; j <= N; ++j) {
-                        Y[j][i] = (i < N) ? dt * M[i * (N + 1) + j] : 0.f;
-                        Wd[i][j] = (i < N) ? lam[i] * q[j] : 0.f;
-                    }
-                frechet_expm<N + 1>(Y, Wd, L, R);
-#pragma unroll
-                for (int i = 0; i < N; ++i)
-#pragma unroll
-                    for (int j = 0; j <= N; ++j)
-                        acc[i * (N + 1) + j] = fmaf(dt, L[i][j], acc[i * (N + 1) + j]);
-                // R = T^T: lambda_prev[k] = sum_r T[r][k] lambda[r]
-                float nl[N];
-#pragma unroll
-                for (int k = 0; k < N; ++k) {
-                    float a = 0.f;
-#pragma unroll
-                    for (int r = 0; r < N; ++r) a = fmaf(R[k][r], lam[r], a);
-                    nl[k] = a;
-                }
+                // the sub-step's start q and the cotangent there
+                float q[N + 1], nl[N];
+                if (norm * dt < kShortStep)
+                    back_step<N, kShortTerms, 2>(M, p, v, lam, dt, acc, q, nl);
+                else
+                    back_step<N, kFlowTerms, 4>(M, p, v, lam, dt, acc, q, nl);
                 float qp[N];
 #pragma unroll
                 for (int r = 0; r < N; ++r) qp[r] = q[r];

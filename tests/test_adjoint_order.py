@@ -66,3 +66,26 @@ def test_fused_backward_walks_every_point(cuda, tmp_path, nc, size, outsize, gra
     b = torch.autograd.grad(ref, [theta, data], w)
     assert (a[0] - b[0]).norm() <= 1e-4 * b[0].norm()
     assert (a[1] - b[1]).norm() <= 1e-5 * b[1].norm()
+
+
+@pytest.mark.parametrize('nc,size', [([3, 3], (40, 12)), ([3, 3], (9, 32)), ([8, 8], (64, 64)),
+                                     ([2, 2, 2], (8, 6, 10)), ([7], (50,))])
+def test_exact_flow_meshgrid_and_shuffled(cuda, nc, size):
+    """The exact flow takes a meshgrid, and its image in the backward, in patches
+    too; a point's flow does not depend on the points beside it."""
+    from libcpab_gb300 import _native as N
+    g = torch.Generator(device=cuda).manual_seed(sum(size))
+    n = len(nc)
+    pts = mesh(cuda, size)
+    nP = pts.shape[1]
+    B = torch.randn(N.num_cells(nc) * n * (n + 1), 5, generator=g, device=cuda)
+    A, _, _ = N.cell_tables(nc, 50, 0.2 * torch.randn(2, 5, generator=g, device=cuda), B)
+    gout = torch.randn(2, n, nP, generator=g, device=cuda)
+    out = N.integrate_exact(nc, pts, A)
+    dth, dp = N.backward_exact(nc, out, A, B, gout, want_dpoints=True)
+    perm = torch.randperm(nP, generator=g, device=cuda)
+    out2 = N.integrate_exact(nc, pts[:, perm].contiguous(), A)
+    dth2, dp2 = N.backward_exact(nc, out2, A, B, gout[:, :, perm].contiguous(), want_dpoints=True)
+    assert torch.equal(out[:, :, perm], out2) and torch.equal(dp[:, :, perm], dp2)
+    assert (dth - dth2).norm() <= 1e-5 * dth2.norm()
+    assert torch.equal(dth, N.backward_exact(nc, out, A, B, gout)[0])
