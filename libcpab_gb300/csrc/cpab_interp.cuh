@@ -142,20 +142,19 @@ __device__ __forceinline__ CornerStep<N> corner_steps(const float (&p)[N], const
 // with m^1 (axis 0), leaving entries indexed by the remaining bits (axis 1 as
 // bit 0), and so on.
 
-// d(lerp)/d(f_j) and the per-corner weights, for the backward passes.
-template <int N>
-__device__ __forceinline__ void lerp_grads(const float *D, const Corner<N> &cr, float w,
-                                           float *ddata_plane, float (&gf)[N]) {
-    float v[1 << N];
-#pragma unroll
-    for (int m = 0; m < (1 << N); ++m) v[m] = __ldg(D + cr.off[m]);
+// d(lerp)/d(f_j) and the per-corner weights, for the backward passes: from the
+// corner values v, the weights f and the cotangent w, gf += and the scatter into
+// d(data), add(m, wt) for corner m.
+template <int N, typename Add>
+__device__ __forceinline__ void lerp_grads_of(const float (&v)[1 << N], const float (&f)[N],
+                                              float w, float (&gf)[N], const Add &add) {
 #pragma unroll
     for (int m = 0; m < (1 << N); ++m) {
         // chain order of autograd: last lerp (highest axis) first
         float wt = w;
 #pragma unroll
-        for (int j = N - 1; j >= 0; --j) wt *= ((m >> j) & 1) ? cr.f[j] : (1.f - cr.f[j]);
-        if (ddata_plane) atomicAdd(ddata_plane + cr.off[m], wt);
+        for (int j = N - 1; j >= 0; --j) wt *= ((m >> j) & 1) ? f[j] : (1.f - f[j]);
+        add(m, wt);
     }
 #pragma unroll
     for (int j = 0; j < N; ++j) {
@@ -167,11 +166,22 @@ __device__ __forceinline__ void lerp_grads(const float *D, const Corner<N> &cr, 
             float wt = 1.f;
 #pragma unroll
             for (int q = 0; q < N; ++q)
-                if (q != j) wt *= ((m >> q) & 1) ? cr.f[q] : (1.f - cr.f[q]);
+                if (q != j) wt *= ((m >> q) & 1) ? f[q] : (1.f - f[q]);
             s = fmaf(wt, v[m | (1 << j)] - v[m], s);
         }
         gf[j] += w * s;
     }
+}
+
+template <int N>
+__device__ __forceinline__ void lerp_grads(const float *D, const Corner<N> &cr, float w,
+                                           float *ddata_plane, float (&gf)[N]) {
+    float v[1 << N];
+#pragma unroll
+    for (int m = 0; m < (1 << N); ++m) v[m] = __ldg(D + cr.off[m]);
+    lerp_grads_of<N>(v, cr.f, w, gf, [&](int m, float wt) {
+        if (ddata_plane) atomicAdd(ddata_plane + cr.off[m], wt);
+    });
 }
 
 inline Geo make_geo(int ndim, const int *size, const int *outsize) {
