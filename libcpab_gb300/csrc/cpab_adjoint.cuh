@@ -660,28 +660,38 @@ __device__ __forceinline__ void reverse_sweep(const AdjSmem<N, CT> &sm, int nste
     reverse_sweep_to<N, MODE, CT>(sm, nsteps, st, lam, sink);
 }
 
+template <int N>
+__device__ __forceinline__ void e_step(const float *tabE, const Tess &t, float (&p)[N],
+                                       unsigned long long *ties) {
+    constexpr int P = N * (N + 1);
+    const int c = find_cell<N>(p, t, ties);
+    float M[P], y[N];
+    load_cell<N>(tabE, c, M);
+    affine_apply<N>(M, p, y);
+#pragma unroll
+    for (int r = 0; r < N; ++r) p[r] += y[r];
+}
+
 // Sweep with the arithmetic of k_integrate's compensated path,
 // p <- p + E_c [p;1], nsteps times.  tabE may be in shared or global memory.
 template <int N>
 __device__ __forceinline__ void e_sweep(const float *tabE, const Tess &t, int nsteps,
                                         float (&p)[N], unsigned long long *ties, unsigned *err) {
-    constexpr int P = N * (N + 1);
-    for (int s = 0; s < nsteps; ++s) {
-        int c = find_cell<N>(p, t, ties);
-        float M[P], y[N];
-        load_cell<N>(tabE, c, M);
-        affine_apply<N>(M, p, y);
-#pragma unroll
-        for (int r = 0; r < N; ++r) p[r] += y[r];
-    }
+    for (int s = 0; s < nsteps; ++s) e_step<N>(tabE, t, p, ties);
 }
 
 // Forward sweep that logs cells and checkpoints; p holds p_0 on entry and
 // p_N on exit.
-template <int N, int MODE, typename CT>
+// beside: another trajectory's step, taken at each of these.
+struct NoStep {
+    __device__ __forceinline__ void operator()() const {}
+};
+
+template <int N, int MODE, typename CT, typename Step = NoStep>
 __device__ __forceinline__ void logged_forward(const AdjSmem<N, CT> &sm, const Tess &t,
                                                int nsteps, const Steps &st, float (&p)[N],
-                                               unsigned long long *ties, unsigned *err) {
+                                               unsigned long long *ties, unsigned *err,
+                                               const Step &beside = Step()) {
     const int B = blockDim.x, tid = threadIdx.x;
     for (int n0 = 0, seg = 0; n0 < nsteps; n0 += kSeg, ++seg) {
 #pragma unroll
@@ -692,6 +702,7 @@ __device__ __forceinline__ void logged_forward(const AdjSmem<N, CT> &sm, const T
             sm.cl[n * B + tid] = (CT)c;
             if constexpr (MODE == 2) mid_map_step<N>(sm.dtab, sm.mtab, c, p);
             else traj_step<N, MODE>(sm.tab, c, st, p);
+            beside();
         }
     }
 }

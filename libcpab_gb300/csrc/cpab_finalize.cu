@@ -33,12 +33,12 @@ constexpr int kFinalizeThreads = 512;
 
 // Where a theta's partials are: `count` rows of G floats from `first`.
 // Dense: [n_theta][parts][G].  Ragged (tile_off != null): set s owns the slots
-// w + s of the warps w that touch it (see cpab_ragged.cuh).
+// v + s of the chunks v that touch it (see cpab_ragged.cuh).
 struct Partials {
     const float *base;
     int parts;
     const int *tile_off;   // [S + 1] or null
-    int S, TW;
+    int S, warps, chunks;  // tile_chunks
 };
 
 __device__ __forceinline__ void partial_rows(const Partials &p, int th, long long *first,
@@ -49,11 +49,11 @@ __device__ __forceinline__ void partial_rows(const Partials &p, int th, long lon
         return;
     }
     const int TT = __ldg(p.tile_off + p.S);
-    const int K = max(1, (TT + p.TW - 1) / p.TW);
+    const TileChunks tc = tile_chunks(TT, p.warps, p.chunks);
     const int a = __ldg(p.tile_off + th), b = __ldg(p.tile_off + th + 1);
-    const int w0 = a / K;
-    *first = (long long)w0 + th;
-    *count = b > a ? (b - 1) / K - w0 + 1 : 0;
+    const int v0 = tc.of(a);
+    *first = (long long)v0 + th;
+    *count = b > a ? tc.of(b - 1) - v0 + 1 : 0;
 }
 
 // Cell statistics g (n cells from A's first row) -> dL/dA in place.
@@ -275,10 +275,10 @@ cudaError_t launch_finalize(const Tess &t, int nsteps, int mode, const float *pa
 }
 
 cudaError_t launch_ragged_finalize(const Tess &t, int nsteps, int mode, const float *partials,
-                                   const int *tile_off, int S, int warps, const float *A,
+                                   const int *tile_off, int S, int warps, int chunks, const float *A,
                                    const float *basis, int d, float *dtheta,
                                    const float *sse_partials, float *sse, cudaStream_t s) {
-    const Partials ps = {partials, 0, tile_off, S, warps};
+    const Partials ps = {partials, 0, tile_off, S, warps, chunks};
     return dispatch(t, nsteps, mode, ps, A, basis, d, S, dtheta, sse_partials, sse, s);
 }
 

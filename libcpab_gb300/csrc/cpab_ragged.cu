@@ -91,7 +91,10 @@ __global__ void __launch_bounds__(1024)
         const long long a = off[s], b = off[s + 1];
         if (series_ok(a, b, total)) run += (b - a + tpw - 1) / tpw;
     }
-    if (tid == B - 1) tile_off[S] = (int)run;
+    if (tid == B - 1) {
+        tile_off[S] = (int)run;
+        tile_off[S + 1] = 0;   // next_chunk's counter
+    }
 }
 
 cudaError_t launch_ragged_plan(int S, const long long *off, long long total, int tpw,
@@ -189,13 +192,13 @@ __host__ __device__ inline size_t ragged_adjoint_smem(int nC, int nsteps, int bl
 
 // The lane-slot sink of the reverse sweep (LS = true): a lane that leaves a
 // cell adds its sum over the steps spent there into its own slots
-// ls[cell][i][lane] with fire-and-forget global reductions, and widens the
+// ls[cell][lane][2] with a fire-and-forget global reduction, and widens the
 // range [lo, hi] of cells it touched.  Each slot is written by one lane only,
 // in program order, so its value does not depend on timing; the warp sums the
 // 32 slots of each touched cell with a fixed shuffle tree when it finishes a
 // series (reproducible dtheta).  Unlike the warp-table flush (a five-round
 // shuffle tree over the run of lanes in a cell, executed by the whole warp at
-// every step where any lane changes cell), a lane's flush is two reductions.
+// every step where any lane changes cell), a lane's flush is one reduction.
 struct LaneSlotSink {
     float *ls;
     int lo, hi;
@@ -204,9 +207,9 @@ struct LaneSlotSink {
     __device__ __forceinline__ void changed(unsigned, bool change, int cell,
                                             const float (&acc)[P]) {
         if (change) {
-            float *q = ls + cell * (P * 32) + (threadIdx.x & 31);
-#pragma unroll
-            for (int i = 0; i < P; ++i) atomicAdd(q + i * 32, acc[i]);
+            static_assert(P == 2);
+            atomicAdd(reinterpret_cast<float2 *>(ls) + cell * 32 + (threadIdx.x & 31),
+                      make_float2(acc[0], acc[1]));
             lo = min(lo, cell);
             hi = max(hi, cell);
         }
@@ -217,7 +220,7 @@ template <int MODE, typename CT, bool FUSED, bool LS>
 __global__ void __launch_bounds__(256)
     k_ragged_adjoint(const __grid_constant__ Tess t,
                      int nsteps, Steps st, int S, const long long *__restrict__ off,
-                     const int *__restrict__ tile_off, int ppt, RaggedBwd a,
+                     int *tile_off, int chunks, int ppt, RaggedBwd a,
                      unsigned long long *ties, unsigned *err) {
     constexpr int P = 2;
     extern __shared__ float4 smem4[];
@@ -240,13 +243,9 @@ __global__ void __launch_bounds__(256)
     const int TW = gridDim.x * W;
     const int w = blockIdx.x * W + wib;
     const int TT = __ldg(tile_off + S);
-    const int K = (TT + TW - 1) / TW;
-    const long long t0 = (long long)w * K;
-    const int t1 = (int)min(t0 + K, (long long)TT);
-    if (t0 >= t1) return;   // warp-uniform; no block-level barrier follows
+    const TileChunks tc = tile_chunks(TT, TW, chunks);
+    if (tc.start(w) >= TT) return;   // warp-uniform; no block-level barrier follows
     const int tpw = 32 * ppt;
-    int s = find_series(tile_off, S, (int)t0);
-    int s_end = __ldg(tile_off + s + 1);
     float sse = 0.f;
     LaneSlotSink slots{LS ? a.lane_slots + (size_t)w * t.nC * (P * 32) : nullptr, INT_MAX, -1};
     if constexpr (LS) {
@@ -265,86 +264,102 @@ __global__ void __launch_bounds__(256)
         build_dtab<1, MODE>(sm.tab, sm.dtab, t.nC, st, lane, 32);
         __syncwarp();
     };
-    auto finish = [&](int sid) {
+    auto finish = [&](int v, int sid) {
         __syncwarp();
         if constexpr (LS) {
             // cell sums of the series into gw; the slots are zeroed for the next one
             const int lo = __reduce_min_sync(0xffffffffu, slots.lo);
             const int hi = __reduce_max_sync(0xffffffffu, slots.hi);
-            for (int c = lo; c <= hi; ++c) {
-                float *q = slots.ls + c * (P * 32) + lane;
-                float v[P];
+            // K cells at a time, their loads in flight together (one by one, each
+            // cell cost an L2 latency: 8 % of the kernel with 1,024 series)
+            constexpr int K = 8;
+            for (int c = lo; c <= hi; c += K) {
+                float2 *q = reinterpret_cast<float2 *>(slots.ls) + c * 32 + lane;
+                float v[K * P];
 #pragma unroll
-                for (int i = 0; i < P; ++i) {
-                    v[i] = __ldcg(q + i * 32);   // this lane's own reductions, in order
-                    q[i * 32] = 0.f;
+                for (int k = 0; k < K; ++k) {
+                    // this lane's own reductions, in order
+                    const float2 u = c + k <= hi ? __ldcg(q + k * 32) : make_float2(0.f, 0.f);
+                    v[2 * k] = u.x;
+                    v[2 * k + 1] = u.y;
                 }
 #pragma unroll
-                for (int d = 16; d > 0; d >>= 1)
-#pragma unroll
-                    for (int i = 0; i < P; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], d);
-                if (lane == 0) {
-#pragma unroll
-                    for (int i = 0; i < P; ++i) sm.gw[c * P + i] = v[i];
-                }
+                for (int k = 0; k < K; ++k)
+                    if (c + k <= hi) q[k * 32] = make_float2(0.f, 0.f);
+                const float sum = warp_sums<K * P>(v, true);
+                const int i = c * P + sum_index<K * P>(lane);
+                if (!(lane & 1) && i < (hi + 1) * P) sm.gw[i] = sum;
             }
             slots.lo = INT_MAX;
             slots.hi = -1;
             __syncwarp();
         }
-        float v = sse;
+        float sum = sse;
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-        const long long slot = (long long)w + sid;
-        if (FUSED && lane == 0) a.sse_partials[slot] = v;
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        const long long slot = (long long)v + sid;
+        if (FUSED && lane == 0) a.sse_partials[slot] = sum;
         for (int i = lane; i < G; i += 32) a.partials[slot * G + i] = sm.gw[i];
         sse = 0.f;
     };
 
-    stage(s);
-    for (int tl = (int)t0; tl < t1; ++tl) {
-        if (tl >= s_end) {
-            finish(s);
-            while (tl >= s_end) s_end = __ldg(tile_off + (++s) + 1);
-            stage(s);
-        }
-        const long long base = __ldg(off + s);
-        const int L = (int)(__ldg(off + s + 1) - base);
-        const float step = (L > 1) ? 1.f / (float)(L - 1) : 0.f;
-        const int j0 = (tl - __ldg(tile_off + s)) * tpw;
-        const Geo g = series_geo(L);
-#pragma unroll 1
-        for (int k = 0; k < ppt; ++k) {
-            const int j = j0 + k * 32 + lane;
-            const bool live = j < L;
-            float p[1] = {live ? linspace01(j, L, step) : 0.5f};
-            float pN[1] = {p[0]};
-            if constexpr (MODE != 1) e_sweep<1>(tabE, t, nsteps, pN, ties, err);
-            logged_forward<1, MODE, CT>(sm, t, nsteps, st, p, ties, err);
-            if constexpr (MODE == 1) pN[0] = p[0];
-            float lam[1] = {0.f};
-            if (live) {
-                const Corner<1> cr = corners<1>(pN, g);
-                float wgt;
-                if constexpr (FUSED) {
-                    const float v = lerp_corners<1>(a.values + base, cr);
-                    if (a.out) a.out[base + j] = v;
-                    const float r = v - __ldg(a.target + base + j);
-                    sse = fmaf(r, r, sse);
-                    wgt = a.loss_scale * r;
-                } else {
-                    wgt = __ldg(a.gout + base + j);
-                }
-                float gf[1] = {0.f};
-                lerp_grads<1>(a.values + base, cr, wgt, a.dvalues ? a.dvalues + base : nullptr,
-                              gf);
-                lam[0] = gf[0] * g.sizem1[0];
+    for (int v = w;;) {
+        const int t0 = (int)tc.start(v), t1 = (int)min(tc.start(v + 1), (long long)TT);
+        int s = find_series(tile_off, S, t0);
+        int s_end = __ldg(tile_off + s + 1);
+        stage(s);
+        for (int tl = t0; tl < t1; ++tl) {
+            if (tl >= s_end) {
+                finish(v, s);
+                while (tl >= s_end) s_end = __ldg(tile_off + (++s) + 1);
+                stage(s);
             }
-            if constexpr (LS) reverse_sweep_to<1, MODE, CT>(sm, nsteps, st, lam, slots);
-            else reverse_sweep<1, MODE, CT, false, true>(sm, nsteps, st, lam, sm.gw);
+            const long long base = __ldg(off + s);
+            const int L = (int)(__ldg(off + s + 1) - base);
+            const float step = (L > 1) ? 1.f / (float)(L - 1) : 0.f;
+            const int j0 = (tl - __ldg(tile_off + s)) * tpw;
+            const Geo g = series_geo(L);
+#pragma unroll 1
+            for (int k = 0; k < ppt; ++k) {
+                const int j = j0 + k * 32 + lane;
+                const bool live = j < L;
+                float p[1] = {live ? linspace01(j, L, step) : 0.5f};
+                float pN[1] = {p[0]};
+                if constexpr (MODE != 1) {
+                    // the two trajectories step by step: two chains in flight
+                    // (4,096 series 1.60 -> 1.55 ms)
+                    logged_forward<1, MODE, CT>(sm, t, nsteps, st, p, ties, err,
+                                                [&] { e_step<1>(tabE, t, pN, ties); });
+                } else {
+                    logged_forward<1, MODE, CT>(sm, t, nsteps, st, p, ties, err);
+                    pN[0] = p[0];
+                }
+                float lam[1] = {0.f};
+                if (live) {
+                    const Corner<1> cr = corners<1>(pN, g);
+                    float wgt;
+                    if constexpr (FUSED) {
+                        const float v = lerp_corners<1>(a.values + base, cr);
+                        if (a.out) a.out[base + j] = v;
+                        const float r = v - __ldg(a.target + base + j);
+                        sse = fmaf(r, r, sse);
+                        wgt = a.loss_scale * r;
+                    } else {
+                        wgt = __ldg(a.gout + base + j);
+                    }
+                    float gf[1] = {0.f};
+                    lerp_grads<1>(a.values + base, cr, wgt, a.dvalues ? a.dvalues + base : nullptr,
+                                  gf);
+                    lam[0] = gf[0] * g.sizem1[0];
+                }
+                if constexpr (LS) reverse_sweep_to<1, MODE, CT>(sm, nsteps, st, lam, slots);
+                else reverse_sweep<1, MODE, CT, false, true>(sm, nsteps, st, lam, sm.gw);
+            }
         }
+        finish(v, s);
+        v = next_chunk(tile_off + S + 1, TW);
+        if (v >= chunks || tc.start(v) >= TT) break;
     }
-    finish(s);
 }
 
 // ------------------------------- planning ------------------------------------
@@ -366,8 +381,8 @@ static size_t lane_slot_bytes(const Tess &t) {
 }
 
 size_t ragged_workspace_bytes(const Tess &t, int S) {
-    const size_t tiles = ((size_t)(S + 1) * 4 + 255) & ~(size_t)255;
-    const size_t slots = (size_t)num_sms() * 64 + (size_t)S;
+    const size_t tiles = tile_off_bytes(S);
+    const size_t slots = (size_t)num_sms() * kChunksPerSM + (size_t)S;
     const size_t part = (slots * t.nC * 2 * 4 + 255) & ~(size_t)255;
     const size_t sse = (slots * 4 + 255) & ~(size_t)255;
     return tiles + part + sse + lane_slot_bytes(t);
@@ -376,8 +391,8 @@ size_t ragged_workspace_bytes(const Tess &t, int S) {
 static void ragged_carve(const Tess &t, int S, void *ws, int **tile_off, float **partials,
                          float **sse_partials, float **lane_slots) {
     char *p = static_cast<char *>(ws);
-    const size_t tiles = ((size_t)(S + 1) * 4 + 255) & ~(size_t)255;
-    const size_t slots = (size_t)num_sms() * 64 + (size_t)S;
+    const size_t tiles = tile_off_bytes(S);
+    const size_t slots = (size_t)num_sms() * kChunksPerSM + (size_t)S;
     const size_t part = (slots * t.nC * 2 * 4 + 255) & ~(size_t)255;
     const size_t sse = (slots * 4 + 255) & ~(size_t)255;
     *tile_off = reinterpret_cast<int *>(p);
@@ -442,7 +457,7 @@ cudaError_t launch_ragged_forward(const Tess &t, int nsteps, int block, int ppt,
 
 template <int MODE, typename CT, bool FUSED, bool LS>
 static cudaError_t launch_ra_ls(const Tess &t, int nsteps, int block, int ppt, int S,
-                                const long long *off, const int *tile_off, const RaggedBwd &a,
+                                const long long *off, int *tile_off, const RaggedBwd &a,
                                 const float *basis, int d, float *dtheta, float *sse,
                                 unsigned long long *ties, unsigned *err, cudaStream_t s) {
     auto kern = k_ragged_adjoint<MODE, CT, FUSED, LS>;
@@ -451,20 +466,19 @@ static cudaError_t launch_ra_ls(const Tess &t, int nsteps, int block, int ppt, i
     if (e != cudaSuccess) return e;
     const int per_sm = resident_blocks((const void *)kern, block, smem);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
-    // partial slots are sized for at most 64 resident warps per SM, lane slots
-    // for kLaneSlotWarpsPerSM
+    // lane slots are sized for kLaneSlotWarpsPerSM resident warps
     const int grid = min(num_sms() * per_sm,
-                         num_sms() * (LS ? kLaneSlotWarpsPerSM : 64) / (block / 32));
+                         num_sms() * (LS ? kLaneSlotWarpsPerSM : kChunksPerSM) / (block / 32));
     const Steps st = make_steps(nsteps);
-    kern<<<grid, block, smem, s>>>(t, nsteps, st, S, off, tile_off, ppt, a, ties, err);
+    const int warps = grid * (block / 32), chunks = num_sms() * kChunksPerSM;
+    kern<<<grid, block, smem, s>>>(t, nsteps, st, S, off, tile_off, chunks, ppt, a, ties, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    return launch_ragged_finalize(t, nsteps, MODE, a.partials, tile_off, S, grid * (block / 32),
-                                  a.A, basis, d, dtheta, a.sse_partials, sse, s);
+    return launch_ragged_finalize(t, nsteps, MODE, a.partials, tile_off, S, warps, chunks, a.A, basis, d, dtheta, a.sse_partials, sse, s);
 }
 
 template <int MODE, typename CT, bool FUSED>
 static cudaError_t launch_ra_t(const Tess &t, int nsteps, int block, int ppt, int S,
-                               const long long *off, const int *tile_off, const RaggedBwd &a,
+                               const long long *off, int *tile_off, const RaggedBwd &a,
                                const float *basis, int d, float *dtheta, float *sse,
                                unsigned long long *ties, unsigned *err, cudaStream_t s) {
     if (a.lane_slots)

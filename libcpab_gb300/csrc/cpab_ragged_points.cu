@@ -22,7 +22,7 @@ template <int N, int PPT>
 __global__ void __launch_bounds__(256)
     k_ragged_points_forward(const __grid_constant__ Tess t,
                             int nsteps, int S, const long long *__restrict__ off,
-                            const int *__restrict__ tile_off, const float *__restrict__ E,
+                            int *tile_off, int chunks, const float *__restrict__ E,
                             long long total, const float *__restrict__ points,
                             float *__restrict__ out, unsigned long long *ties, unsigned *err) {
     constexpr int P = N * (N + 1);
@@ -34,51 +34,54 @@ __global__ void __launch_bounds__(256)
     const int TW = gridDim.x * (blockDim.x >> 5);
     const int w = blockIdx.x * (blockDim.x >> 5) + wib;
     const int TT = __ldg(tile_off + S);
-    const int K = (TT + TW - 1) / TW;
-    const long long t0 = (long long)w * K;
-    const int t1 = (int)min(t0 + K, (long long)TT);
-    if (t0 >= t1) return;
-    int s = find_series(tile_off, S, (int)t0);
-    int s_end = __ldg(tile_off + s + 1);
-    bool staged = false;
-    for (int tl = (int)t0; tl < t1; ++tl) {
-        if (tl >= s_end || !staged) {
+    const TileChunks tc = tile_chunks(TT, TW, chunks);
+    if (tc.start(w) >= TT) return;
+    int staged = -1;
+    for (int v = w;;) {
+        const int t0 = (int)tc.start(v), t1 = (int)min(tc.start(v + 1), (long long)TT);
+        int s = find_series(tile_off, S, t0);
+        int s_end = __ldg(tile_off + s + 1);
+        for (int tl = t0; tl < t1; ++tl) {
             while (tl >= s_end) s_end = __ldg(tile_off + (++s) + 1);
-            __syncwarp();
-            for (int i = lane; i < G; i += 32) tab[i] = __ldg(E + (long long)s * G + i);
-            __syncwarp();
-            staged = true;
-        }
-        const long long base = __ldg(off + s);
-        const int L = (int)(__ldg(off + s + 1) - base);
-        const int j0 = (tl - __ldg(tile_off + s)) * TPW;
-        float p[PPT][N];
-        int j[PPT];
-#pragma unroll
-        for (int k = 0; k < PPT; ++k) {
-            j[k] = j0 + k * 32 + lane;
-#pragma unroll
-            for (int r = 0; r < N; ++r)
-                p[k][r] = (j[k] < L) ? __ldg(points + r * total + base + j[k]) : 0.5f;
-        }
-        for (int st = 0; st < nsteps; ++st) {
-            int c[PPT];
-            find_cells<N, PPT>(p, c, t, ties);
+            if (s != staged) {
+                __syncwarp();
+                for (int i = lane; i < G; i += 32) tab[i] = __ldg(E + (long long)s * G + i);
+                __syncwarp();
+                staged = s;
+            }
+            const long long base = __ldg(off + s);
+            const int L = (int)(__ldg(off + s + 1) - base);
+            const int j0 = (tl - __ldg(tile_off + s)) * TPW;
+            float p[PPT][N];
+            int j[PPT];
 #pragma unroll
             for (int k = 0; k < PPT; ++k) {
-                float M[P], y[N];
-                load_cell<N>(tab, c[k], M);
-                affine_apply<N>(M, p[k], y);
+                j[k] = j0 + k * 32 + lane;
 #pragma unroll
-                for (int r = 0; r < N; ++r) p[k][r] += y[r];
+                for (int r = 0; r < N; ++r)
+                    p[k][r] = (j[k] < L) ? __ldg(points + r * total + base + j[k]) : 0.5f;
+            }
+            for (int st = 0; st < nsteps; ++st) {
+                int c[PPT];
+                find_cells<N, PPT>(p, c, t, ties);
+#pragma unroll
+                for (int k = 0; k < PPT; ++k) {
+                    float M[P], y[N];
+                    load_cell<N>(tab, c[k], M);
+                    affine_apply<N>(M, p[k], y);
+#pragma unroll
+                    for (int r = 0; r < N; ++r) p[k][r] += y[r];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < PPT; ++k) {
+                if (j[k] >= L) continue;
+#pragma unroll
+                for (int r = 0; r < N; ++r) out[r * total + base + j[k]] = p[k][r];
             }
         }
-#pragma unroll
-        for (int k = 0; k < PPT; ++k) {
-            if (j[k] >= L) continue;
-#pragma unroll
-            for (int r = 0; r < N; ++r) out[r * total + base + j[k]] = p[k][r];
-        }
+        v = next_chunk(tile_off + S + 1, TW);
+        if (v >= chunks || tc.start(v) >= TT) break;
     }
 }
 
@@ -102,7 +105,7 @@ template <int N, int MODE, typename CT>
 __global__ void __launch_bounds__(256, 3)
     k_ragged_points_adjoint(const __grid_constant__ Tess t,
                             int nsteps, Steps st, int S, const long long *__restrict__ off,
-                            const int *__restrict__ tile_off, int ppt,
+                            int *tile_off, int chunks, int ppt,
                             const float *__restrict__ table, long long total,
                             const float *__restrict__ points, const float *__restrict__ gout,
                             float *__restrict__ dpoints, float *__restrict__ partials,
@@ -127,13 +130,9 @@ __global__ void __launch_bounds__(256, 3)
     const int TW = gridDim.x * W;
     const int w = blockIdx.x * W + wib;
     const int TT = __ldg(tile_off + S);
-    const int K = (TT + TW - 1) / TW;
-    const long long t0 = (long long)w * K;
-    const int t1 = (int)min(t0 + K, (long long)TT);
-    if (t0 >= t1) return;   // warp-uniform; no block-level barrier follows
+    const TileChunks tc = tile_chunks(TT, TW, chunks);
+    if (tc.start(w) >= TT) return;   // warp-uniform; no block-level barrier follows
     const int tpw = 32 * ppt;
-    int s = find_series(tile_off, S, (int)t0);
-    int s_end = __ldg(tile_off + s + 1);
 
     auto stage = [&](int sid) {
         __syncwarp();
@@ -144,61 +143,68 @@ __global__ void __launch_bounds__(256, 3)
         build_dtab<N, MODE>(sm.tab, sm.dtab, t.nC, st, lane, 32);
         __syncwarp();
     };
-    auto finish = [&](int sid) {
+    auto finish = [&](int v, int sid) {
         __syncwarp();
-        const long long slot = (long long)w + sid;
+        const long long slot = (long long)v + sid;
         for (int i = lane; i < G; i += 32) partials[slot * G + i] = sm.gw[i];
     };
 
-    stage(s);
-    for (int tl = (int)t0; tl < t1; ++tl) {
-        if (tl >= s_end) {
-            finish(s);
-            while (tl >= s_end) s_end = __ldg(tile_off + (++s) + 1);
-            stage(s);
-        }
-        const long long base = __ldg(off + s);
-        const int L = (int)(__ldg(off + s + 1) - base);
-        const int j0 = (tl - __ldg(tile_off + s)) * tpw;
+    for (int v = w;;) {
+        const int t0 = (int)tc.start(v), t1 = (int)min(tc.start(v + 1), (long long)TT);
+        int s = find_series(tile_off, S, t0);
+        int s_end = __ldg(tile_off + s + 1);
+        stage(s);
+        for (int tl = t0; tl < t1; ++tl) {
+            if (tl >= s_end) {
+                finish(v, s);
+                while (tl >= s_end) s_end = __ldg(tile_off + (++s) + 1);
+                stage(s);
+            }
+            const long long base = __ldg(off + s);
+            const int L = (int)(__ldg(off + s + 1) - base);
+            const int j0 = (tl - __ldg(tile_off + s)) * tpw;
 #pragma unroll 1
-        for (int k = 0; k < ppt; ++k) {
-            const int j = j0 + k * 32 + lane;
-            const bool live = j < L;
-            float p[N], lam[N];
+            for (int k = 0; k < ppt; ++k) {
+                const int j = j0 + k * 32 + lane;
+                const bool live = j < L;
+                float p[N], lam[N];
 #pragma unroll
-            for (int r = 0; r < N; ++r) {
-                p[r] = live ? __ldg(points + r * total + base + j) : 0.5f;
-                lam[r] = live ? __ldg(gout + r * total + base + j) : 0.f;
-            }
-            logged_forward<N, MODE, CT>(sm, t, nsteps, st, p, ties, err);
-            reverse_sweep<N, MODE, CT, false, true>(sm, nsteps, st, lam, sm.gw);
-            if (dpoints && live) {
+                for (int r = 0; r < N; ++r) {
+                    p[r] = live ? __ldg(points + r * total + base + j) : 0.5f;
+                    lam[r] = live ? __ldg(gout + r * total + base + j) : 0.f;
+                }
+                logged_forward<N, MODE, CT>(sm, t, nsteps, st, p, ties, err);
+                reverse_sweep<N, MODE, CT, false, true>(sm, nsteps, st, lam, sm.gw);
+                if (dpoints && live) {
 #pragma unroll
-                for (int r = 0; r < N; ++r) dpoints[r * total + base + j] = lam[r];
+                    for (int r = 0; r < N; ++r) dpoints[r * total + base + j] = lam[r];
+                }
             }
         }
+        finish(v, s);
+        v = next_chunk(tile_off + S + 1, TW);
+        if (v >= chunks || tc.start(v) >= TT) break;
     }
-    finish(s);
 }
 
 // ------------------------------- host side -----------------------------------
 size_t ragged_points_workspace_bytes(const Tess &t, int S) {
-    const size_t tiles = ((size_t)(S + 1) * 4 + 255) & ~(size_t)255;
-    const size_t slots = (size_t)num_sms() * 64 + (size_t)S;
+    const size_t tiles = tile_off_bytes(S);
+    const size_t slots = (size_t)num_sms() * kChunksPerSM + (size_t)S;
     const size_t P = (size_t)t.ndim * (t.ndim + 1);
     return tiles + ((slots * t.nC * P * 4 + 255) & ~(size_t)255);
 }
 
 static void points_carve(int S, void *ws, int **tile_off, float **partials) {
     char *p = static_cast<char *>(ws);
-    const size_t tiles = ((size_t)(S + 1) * 4 + 255) & ~(size_t)255;
+    const size_t tiles = tile_off_bytes(S);
     *tile_off = reinterpret_cast<int *>(p);
     *partials = reinterpret_cast<float *>(p + tiles);
 }
 
 template <int N, int PPT>
 static cudaError_t launch_rpf_t(const Tess &t, int nsteps, int S, const long long *off,
-                                const int *tile_off, const float *E, long long total,
+                                int *tile_off, const float *E, long long total,
                                 const float *points, float *out, unsigned long long *ties,
                                 unsigned *err, cudaStream_t s, int block) {
     auto kern = k_ragged_points_forward<N, PPT>;
@@ -206,14 +212,15 @@ static cudaError_t launch_rpf_t(const Tess &t, int nsteps, int S, const long lon
     if (const cudaError_t e = allow_smem((const void *)kern, smem)) return e;
     const int per_sm = resident_blocks((const void *)kern, block, smem);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
-    kern<<<num_sms() * per_sm, block, smem, s>>>(t, nsteps, S, off, tile_off, E, total, points,
-                                                  out, ties, err);
+    const int grid = num_sms() * per_sm;
+    kern<<<grid, block, smem, s>>>(t, nsteps, S, off, tile_off, grid * (block / 32) * kForwardChunks,
+                                   E, total, points, out, ties, err);
     return cudaGetLastError();
 }
 
 template <int N>
 static cudaError_t launch_rpf_n(int ppt, const Tess &t, int nsteps, int S, const long long *off,
-                                const int *tile_off, const float *E, long long total,
+                                int *tile_off, const float *E, long long total,
                                 const float *points, float *out, unsigned long long *ties,
                                 unsigned *err, cudaStream_t s, int block) {
     switch (ppt) {
@@ -270,7 +277,7 @@ static int points_block(const Tess &t, int nsteps, int force_block) {
 
 template <int N, int MODE, typename CT>
 static cudaError_t launch_rpa_t(const Tess &t, int nsteps, int S, const long long *off,
-                                const int *tile_off, const float *A, const float *E,
+                                int *tile_off, const float *A, const float *E,
                                 long long total, const float *points, const float *gout,
                                 float *dpoints, float *partials, const float *basis, int d,
                                 float *dtheta, unsigned long long *ties, unsigned *err,
@@ -284,15 +291,15 @@ static cudaError_t launch_rpa_t(const Tess &t, int nsteps, int S, const long lon
     const int per_sm = resident_blocks((const void *)kern, block, smem);
     if (per_sm <= 0) return cudaErrorInvalidConfiguration;
     const int W = block / 32;
-    // partial slots are sized for at most 64 resident warps per SM
-    const int grid = min(num_sms() * per_sm, num_sms() * 64 / W);
+    const int grid = min(num_sms() * per_sm, num_sms() * kChunksPerSM / W);
     const Steps st = make_steps(nsteps);
-    kern<<<grid, block, smem, s>>>(t, nsteps, st, S, off, tile_off, 1,
+    const int chunks = num_sms() * kChunksPerSM;
+    kern<<<grid, block, smem, s>>>(t, nsteps, st, S, off, tile_off, chunks, 1,
                                    MODE == 1 ? E : A, total, points, gout, dpoints, partials,
                                    ties, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (d == 0 || !dtheta) return cudaSuccess;
-    return launch_ragged_finalize(t, nsteps, MODE, partials, tile_off, S, grid * W, A, basis, d,
+    return launch_ragged_finalize(t, nsteps, MODE, partials, tile_off, S, grid * W, chunks, A, basis, d,
                                   dtheta, nullptr, nullptr, s);
 }
 
