@@ -51,9 +51,9 @@ __device__ __forceinline__ void partial_rows(const Partials &p, int th, long lon
     const int TT = __ldg(p.tile_off + p.S);
     const TileChunks tc = tile_chunks(TT, p.warps, p.chunks);
     const int a = __ldg(p.tile_off + th), b = __ldg(p.tile_off + th + 1);
-    const int v0 = tc.of(a);
+    const unsigned v0 = tc.of((unsigned)a);
     *first = (long long)v0 + th;
-    *count = b > a ? tc.of(b - 1) - v0 + 1 : 0;
+    *count = b > a ? (int)(tc.of((unsigned)(b - 1)) - v0) + 1 : 0;
 }
 
 // Cell statistics g (n cells from A's first row) -> dL/dA in place.

@@ -199,12 +199,14 @@ cudaError_t launch_adjoint_exact(const Tess &t, const AdjointPlan &plan, const f
 // Contiguous chunks of the ragged adjoints' warp tiles, one partial sum per chunk
 // and set: `first` chunks of K1 tiles, then chunks of K2.
 struct TileChunks {
-    long long first, K1, K2;
-    __host__ __device__ long long start(long long v) const {
-        return v < first ? v * K1 : first * K1 + (v - first) * K2;
+    unsigned first, K1, K2;
+    __host__ __device__ long long start(unsigned v) const {
+        return v < first ? (long long)v * K1
+                         : (long long)first * K1 + (long long)(v - first) * K2;
     }
-    __host__ __device__ int of(long long tile) const {
-        return (int)(tile < first * K1 ? tile / K1 : first + (tile - first * K1) / K2);
+    __host__ __device__ unsigned of(unsigned tile) const {
+        const long long low = (long long)first * K1;
+        return tile < low ? tile / K1 : first + (unsigned)(tile - low) / K2;
     }
 };
 
@@ -215,15 +217,15 @@ struct TileChunks {
 // others in small ones: series adjoint (4,096 series) 1.56 -> 1.30 ms, point sets
 // (1,024) 2.54 -> 2.29 ms, 24 mixed images 0.40 -> 0.36 ms; with three fifths 1.31,
 // 2.35 and 0.36 ms, with two fifths and twice the chunks 1.34, 2.39 and 0.35 ms.
-__host__ __device__ inline TileChunks tile_chunks(long long total, long long warps,
-                                                  long long chunks) {
+__host__ __device__ inline TileChunks tile_chunks(unsigned total, unsigned warps,
+                                                  unsigned chunks) {
     TileChunks c;
     c.first = warps;
-    const long long share = chunks > warps ? (total + 1) / 2 : total;
+    const unsigned share = chunks > warps ? (total + 1) / 2 : total;
     c.K1 = (share + warps - 1) / warps;
     c.K1 += c.K1 < 1;
-    const long long rest = total - warps * c.K1;
-    c.K2 = rest > 0 ? (rest + (chunks - warps) - 1) / (chunks - warps) : 1;
+    const long long rest = (long long)total - (long long)warps * c.K1;
+    c.K2 = rest > 0 ? ((unsigned)rest + (chunks - warps) - 1) / (chunks - warps) : 1;
     return c;
 }
 
