@@ -93,15 +93,18 @@ cudaError_t launch_integrate(const Tess &t, int nsteps, const float *points, int
                              long long nP, const float *table, bool compensated, int n_theta,
                              float *out, int *trace, unsigned long long *ties, unsigned *err,
                              cudaStream_t s, const LaunchShape *force) {
-    // Default: 256 threads, two points per thread once there is enough work
-    // to fill the GPU twice; or the autotuned / forced shape.
+    // Default: forward_block threads, two points per thread once there is enough
+    // work to fill the GPU twice, in 2D six times (3.2 M points 0.244 against 0.259
+    // ms with one, 0.8 M points 0.081 against 0.076); or the autotuned / forced
+    // shape.
     LaunchShape sh;
     if (force) {
         sh = *force;
     } else if (!tuned_get(kTuneIntegrate, tune_key(t, nsteps, compensated ? 1 : 0, nP, n_theta,
                                                    broadcast), &sh)) {
-        sh.block = 256;
-        sh.ppt = (long long)n_theta * nP >= (long long)num_sms() * 2048 * 2 ? 2 : 1;
+        sh.block = forward_block(t);
+        sh.ppt = (long long)n_theta * nP >=
+                         (long long)num_sms() * 2048 * (t.ndim == 2 ? 6 : 2) ? 2 : 1;
     }
     if (sh.block < 32 || sh.block > 256 || sh.block % 32 || (sh.ppt != 1 && sh.ppt != 2))
         return cudaErrorInvalidConfiguration;

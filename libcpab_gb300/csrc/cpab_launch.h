@@ -45,6 +45,13 @@ void tuned_clear();
 template <int N>
 __host__ __device__ constexpr int step_blocks() { return N == 1 ? 1 : N == 2 ? 4 : 2; }
 
+// Threads per block of the forward kernels: 128, whose slots free up sooner than
+// those of 256 (transform_grid on 8 x 128^3, [4,4,4], 3.09 against 3.37 ms; 2D 1 %),
+// as long as the tables of all blocks that the registers allow fit in shared memory.
+inline int forward_block(const Tess &t) {
+    return (size_t)t.nC * t.ndim * (t.ndim + 1) * 4 <= 24 * 1024 ? 128 : 256;
+}
+
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) where a launch needs it (near
 // or above 48 KB), once per kernel, device and size; and the occupancy query, kept
 // per kernel, device, block and size.  Both cost microseconds of host time, on
