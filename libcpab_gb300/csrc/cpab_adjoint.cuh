@@ -206,11 +206,11 @@ __host__ __device__ inline size_t adjoint_smem_bytes(int nC, int nsteps, int blo
 // Host: the launch shape of an adjoint kernel with the most resident warps per
 // SM among 256/128/64 threads per CTA and per-warp tables in shared memory
 // (kern_shared) or in global memory (kern_global, may be nullptr; see
-// carve_adjoint), where a warp counts seven eighths: its
-// flushes wait for L2.  [4,4], 64 x 224^2: 0.99 ms with 28 warps in shared memory,
-// 1.04 ms with 32 in global memory; 13 x 151 x 203, exact mode, 0.139 and 0.155 ms;
-// [4,5] 1.34 (shared, 24 warps) and 1.32 ms, [5,5] 1.05 (24) and 1.04 ms.
-// Ties keep shared memory and the larger CTA.  force_block
+// carve_adjoint), where a warp counts seven eighths: its flushes wait for L2.
+// [4,4], 64 x 224^2: 0.99 ms with 28 warps in shared memory, 1.04 ms with 32 in
+// global memory; 13 x 151 x 203, exact mode, 0.139 and 0.155 ms; [4,5] 1.34
+// (shared, 24 warps) and 1.32 ms, [5,5] 1.05 (24) and 1.04 ms.  Ties keep shared
+// memory and the larger CTA.  force_block
 // (> 0) and force_staging (0 shared, 1 global; -1 either) restrict the
 // candidates (the autotuner's shapes).
 template <int N, typename CT, typename K>
