@@ -83,11 +83,13 @@ __device__ float exact_flow_1d(float x, const float *tab, const Tess &t, unsigne
 
 // Conservative distance (domain units) from p to the face lines of its
 // cell's square/cube and to the sub-cell diagonals/planes; the domain
-// boundary is excluded (edge cells extend past it).
+// boundary is excluded (edge cells extend past it).  A single cell in 1D has no
+// face: 1e15 stands for that, so that a step is bounded by 1 / |A| all the same,
+// which the series and the quadrature of a step rest on.
 template <int N>
 __device__ __forceinline__ float face_distance(const float (&p)[N], const Tess &t) {
     float sub[N];
-    float d = INFINITY;
+    float d = 1e15f;
     float imin = t.inc[0];
 #pragma unroll
     for (int j = 0; j < N; ++j) {
