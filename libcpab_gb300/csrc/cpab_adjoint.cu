@@ -80,11 +80,12 @@ __global__ void __launch_bounds__(256, step_blocks<N>())
     float *warp_tab = sm.gw + (size_t)(tid >> 5) * round4(G);
 
     for (int tile = part; tile < tiles; tile += parts) {
-        const bool live = (long long)tile * B + tid < nP;
-        const long long idx = ordered_point((long long)tile * B + tid, order);
+        const long long v = (long long)tile * B + tid;
+        const bool live = v < nP;
+        const long long idx = ordered_point(live ? v : nP - 1, order);
         float p[N], lam[N];
 #pragma unroll
-        for (int r = 0; r < N; ++r) p[r] = live ? __ldg(src + r * nP + idx) : 0.5f;
+        for (int r = 0; r < N; ++r) p[r] = __ldg(src + r * nP + idx);
         logged_forward<N, MODE, CT>(sm, t, nsteps, st, p, ties, err);
 #pragma unroll
         for (int r = 0; r < N; ++r) lam[r] = live ? __ldg(gout + ((long long)th * N + r) * nP + idx) : 0.f;

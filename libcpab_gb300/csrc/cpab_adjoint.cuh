@@ -600,8 +600,10 @@ struct WarpTabSink {
 };
 
 // Reverse sweep of one trajectory whose cells are logged in cl and whose
-// checkpoints are in ck; lam holds dL/dp_N on entry (0 for a lane without a
-// point, whose sums are then zeros) and dL/dp_0 on exit.
+// checkpoints are in ck; lam holds dL/dp_N on entry and dL/dp_0 on exit.  A lane
+// without a point walks with lam = 0 from a point that another lane of the theta
+// has: its sums are zeros unless that trajectory overflows (0 * inf is NaN), and
+// then that lane's are not finite either.
 // Each segment's positions are rebuilt from its checkpoint with the logged
 // cells (no lookups) into pb, then walked backwards.  The loops are not
 // unrolled: the body stays small enough for the instruction cache (unrolled by

@@ -249,10 +249,12 @@ __global__ void __launch_bounds__(256, step_blocks<N>())
         const int o = patch_point<N>(tile * B + tid, patch, g);
         const bool live = o >= 0;
         float p[N], pN[N], lam[N];
+        if (!__any_sync(0xffffffffu, live)) continue;   // the first lane has a point if any has
         if (live) grid_point<N>(o, g, lin, p);
-        else {
 #pragma unroll
-            for (int r = 0; r < N; ++r) p[r] = 0.5f;
+        for (int r = 0; r < N; ++r) {   // lanes without a point follow it
+            const float first = __shfl_sync(0xffffffffu, p[r], 0);
+            if (!live) p[r] = first;
         }
         // composition: the transformations before this one move the grid first
 #pragma unroll

@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(256)
             for (int k = 0; k < ppt; ++k) {
                 const int j = j0 + k * 32 + lane;
                 const bool live = j < L;
-                float p[1] = {live ? linspace01(j, L, step) : 0.5f};
+                float p[1] = {linspace01(min(j, L - 1), L, step)};
                 float pN[1] = {p[0]};
                 if constexpr (MODE != 1) {
                     // the two trajectories step by step: two chains in flight

@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(256, 3)
                 float p[N], lam[N];
 #pragma unroll
                 for (int r = 0; r < N; ++r) {
-                    p[r] = live ? __ldg(points + r * total + base + j) : 0.5f;
+                    p[r] = __ldg(points + r * total + base + min(j, L - 1));
                     lam[r] = live ? __ldg(gout + r * total + base + j) : 0.f;
                 }
                 logged_forward<N, MODE, CT>(sm, t, nsteps, st, p, ties, err);
