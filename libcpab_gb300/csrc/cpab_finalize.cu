@@ -30,6 +30,9 @@ namespace cpab {
 namespace cg = cooperative_groups;
 
 constexpr int kFinalizeThreads = 512;
+// Columns of dtheta per launch: their share of a CTA is held in 32 KB of shared memory.
+// Bases in use have some hundreds; wider ones take a launch for each slice.
+constexpr int kFinalizeColumns = 8192;
 
 // Where a theta's partials are: `count` rows of G floats from `first`.
 // Dense: [n_theta][parts][G].  Ragged (tile_off != null): set s owns the slots
@@ -126,10 +129,11 @@ __device__ __forceinline__ float strided_sum(const float *__restrict__ src, int 
     return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
 }
 
+// d columns from basis and dtheta on, of rows of ld.
 template <int N, int MODE>
 __global__ void __launch_bounds__(kFinalizeThreads)
     k_finalize(int nC, int cells, Steps st, Partials ps, const float *__restrict__ A,
-               const float *__restrict__ basis, int d, float *__restrict__ dtheta,
+               const float *__restrict__ basis, int d, int ld, float *__restrict__ dtheta,
                const float *__restrict__ sse_partials, float *__restrict__ sse) {
     constexpr int P = N * (N + 1);
     extern __shared__ float4 smem4[];
@@ -168,20 +172,28 @@ __global__ void __launch_bounds__(kFinalizeThreads)
     __syncthreads();
     map_cells<N, MODE>(g, A + (long long)th * G + c0 * P, c1 - c0, st);
     // rows of the basis, `split` threads on each column of dtheta
-    const float *b = basis + (long long)c0 * P * d;
+    const float *b = basis + (long long)c0 * P * ld;
     const int split = d <= B ? B / d : 1;
     for (int k0 = 0; k0 < d; k0 += B) {
         const int k = k0 + (d <= B ? tid % d : tid), r0 = d <= B ? tid / d : 0;
         float s[4] = {0.f, 0.f, 0.f, 0.f};
         if (k < d && r0 < split) {
             int i = r0;
+            // 16 loads in flight, added in the same order as four by four
+            for (; i + 15 * split < rows; i += 16 * split) {
+                float v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) v[u] = __ldg(b + (long long)(i + u * split) * ld + k);
+#pragma unroll
+                for (int u = 0; u < 16; ++u) s[u & 3] = fmaf(v[u], g[i + u * split], s[u & 3]);
+            }
             for (; i + 3 * split < rows; i += 4 * split)
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
-                    s[u] = fmaf(__ldg(b + (long long)(i + u * split) * d + k), g[i + u * split],
+                    s[u] = fmaf(__ldg(b + (long long)(i + u * split) * ld + k), g[i + u * split],
                                 s[u]);
             for (; i < rows; i += split)
-                s[0] = fmaf(__ldg(b + (long long)i * d + k), g[i], s[0]);
+                s[0] = fmaf(__ldg(b + (long long)i * ld + k), g[i], s[0]);
         }
         const float v = (s[0] + s[1]) + (s[2] + s[3]);
         if (split == 1) {
@@ -197,22 +209,22 @@ __global__ void __launch_bounds__(kFinalizeThreads)
         }
     }
     if (K == 1) {   // each thread wrote the entries it stores
-        for (int k = tid; k < d; k += B) dtheta[(long long)th * d + k] = dth[k];
+        for (int k = tid; k < d; k += B) dtheta[(long long)th * ld + k] = dth[k];
         return;
     }
     cluster.sync();   // every slice's share is in place
     for (int k = rank * B + tid; k < d; k += K * B) {
         float acc = 0.f;
         for (int q = 0; q < K; ++q) acc += cluster.map_shared_rank(dth, q)[k];
-        dtheta[(long long)th * d + k] = acc;
+        dtheta[(long long)th * ld + k] = acc;
     }
     cluster.sync();   // no CTA leaves while its shared memory is read
 }
 
 template <int N, int MODE>
-static cudaError_t launch_finalize_t(int nC, const Steps &st, const Partials &ps, const float *A,
-                                     const float *basis, int d, int n, float *dtheta,
-                                     const float *sse_partials, float *sse, cudaStream_t s) {
+static cudaError_t launch_columns(int nC, const Steps &st, const Partials &ps, const float *A,
+                                  const float *basis, int d, int ld, int n, float *dtheta,
+                                  const float *sse_partials, float *sse, cudaStream_t s) {
     constexpr int P = N * (N + 1);
     int K = 1, max_optin = 48 * 1024;
     auto bytes = [&](int k) {
@@ -244,8 +256,21 @@ static cudaError_t launch_finalize_t(int nC, const Steps &st, const Partials &ps
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, nC, (nC + K - 1) / K, st, ps, A, basis, d, dtheta,
+    return cudaLaunchKernelEx(&cfg, kern, nC, (nC + K - 1) / K, st, ps, A, basis, d, ld, dtheta,
                               sse_partials, sse);
+}
+
+template <int N, int MODE>
+static cudaError_t launch_finalize_t(int nC, const Steps &st, const Partials &ps, const float *A,
+                                     const float *basis, int d, int n, float *dtheta,
+                                     const float *sse_partials, float *sse, cudaStream_t s) {
+    for (int k = 0;;) {
+        const cudaError_t e = launch_columns<N, MODE>(
+            nC, st, ps, A, basis + k, std::min(d - k, kFinalizeColumns), d, n,
+            dtheta ? dtheta + k : nullptr, sse_partials, k ? nullptr : sse, s);
+        k += kFinalizeColumns;
+        if (e != cudaSuccess || !dtheta || k >= d) return e;
+    }
 }
 
 static cudaError_t dispatch(const Tess &t, int nsteps, int mode, const Partials &ps,
