@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(kFinalizeThreads)
                const float *__restrict__ sse_partials, float *__restrict__ sse) {
     constexpr int P = N * (N + 1);
     extern __shared__ float4 smem4[];
+    __shared__ float sse_s[kFinalizeThreads / 32];
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), K = (int)cluster.num_blocks();
     const int th = blockIdx.x / K, tid = threadIdx.x, B = blockDim.x;
@@ -150,12 +151,26 @@ __global__ void __launch_bounds__(kFinalizeThreads)
     int count;
     partial_rows(ps, th, &first, &count);
     const float *src = ps.base + first * G + c0 * P;
-    if (sse && rank == 0 && tid == 0) {
-        float acc = 0.f;
-        for (int q = 0; q < count; ++q) acc += __ldg(sse_partials + first + q);
-        sse[th] = acc;
+    // the squared error: the chunks' sums over the whole block, in a fixed order (one
+    // thread took up to 10,000 of them one after the other where a series is long)
+    const bool squared = sse && rank == 0;
+    if (squared) {
+        float v = strided_sum(sse_partials + first, tid, B, count, 1);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (!(tid & 31)) sse_s[tid >> 5] = v;
     }
-    if (!dtheta || d <= 0) return;   // uniform over the cluster
+    auto store_sse = [&] {   // after a barrier
+        if (!squared || tid) return;
+        float acc = 0.f;
+        for (int q = 0; q < kFinalizeThreads / 32; ++q) acc += sse_s[q];
+        sse[th] = acc;
+    };
+    if (!dtheta || d <= 0) {   // uniform over the cluster
+        __syncthreads();
+        store_sse();
+        return;
+    }
     // columns of the partials, `split` threads on each
     if (rows > 0 && 2 * rows <= B) {
         const int split = B / rows, i = tid % rows, q0 = tid / rows;
@@ -170,6 +185,7 @@ __global__ void __launch_bounds__(kFinalizeThreads)
         for (int i = tid; i < rows; i += B) g[i] = strided_sum(src + i, 0, 1, count, G);
     }
     __syncthreads();
+    store_sse();
     map_cells<N, MODE>(g, A + (long long)th * G + c0 * P, c1 - c0, st);
     // rows of the basis, `split` threads on each column of dtheta
     const float *b = basis + (long long)c0 * P * ld;
