@@ -56,9 +56,15 @@ def settings(params, device):
 
 
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
-_functorch_level = torch._C._functorch.peek_interpreter_stack
-_function_modes = torch._C._len_torch_function_stack
-_dispatch_modes = torch._C._len_torch_dispatch_stack
+try:
+    _functorch_level = torch._C._functorch.peek_interpreter_stack
+    _function_modes = torch._C._len_torch_function_stack
+    _dispatch_modes = torch._C._len_torch_dispatch_stack
+    _forward_ad = torch.autograd.forward_ad
+    _forward_ad._current_level
+    _tracing = torch._C._get_tracing_state
+except AttributeError:   # a torch that cannot be asked: the Python classes take all calls
+    _PLAIN = ()
 
 
 def native(*tensors):
@@ -69,8 +75,7 @@ def native(*tensors):
         if type(t) not in _PLAIN:
             return False
     return (_functorch_level() is None and _function_modes() == 0 and _dispatch_modes() == 0
-            and torch.autograd.forward_ad._current_level < 0
-            and torch._C._get_tracing_state() is None)
+            and _forward_ad._current_level < 0 and _tracing() is None)
 
 
 class TransformGrid(torch.autograd.Function):

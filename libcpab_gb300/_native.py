@@ -126,26 +126,38 @@ def load(path: str | None = None):
         return lib
 
 
-_bind = None
+_bind = None   # the torch extension, or False where it does not load
+
+
+def _load_bind():
+    from .build import bind_path
+    path = bind_path()
+    try:
+        if not os.path.exists(path):
+            raise ImportError('%s not found; build it with "python -m libcpab_gb300.build"' % path)
+        import importlib.util
+        spec = importlib.util.spec_from_file_location('libcpab_gb300._torch_bind', path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        return mod
+    except ImportError as e:
+        import warnings
+        warnings.warn('the torch extension of libcpab_gb300 does not load, its Python classes '
+                      'take all calls (more host time per call): %s' % e, RuntimeWarning)
+        return False
 
 
 def bind():
-    """The torch extension _torch_bind (native autograd nodes), loaded once."""
+    """The torch extension _torch_bind (native autograd nodes), loaded once, or
+    None (with one warning) where there is none for this torch and Python: the
+    autograd classes in Python make the same calls of the C ABI."""
     global _bind
     if _bind is None:
         load()   # its own message if the C ABI library is missing
         with _lock:
             if _bind is None:
-                path = os.path.join(HERE, '_torch_bind.so')
-                if not os.path.exists(path):
-                    raise ImportError('libcpab_gb300 torch extension not found at %s; build it '
-                                      'with "python -m libcpab_gb300.build"' % path)
-                import importlib.util
-                spec = importlib.util.spec_from_file_location('libcpab_gb300._torch_bind', path)
-                mod = importlib.util.module_from_spec(spec)
-                spec.loader.exec_module(mod)
-                _bind = mod
-    return _bind
+                _bind = _load_bind()
+    return _bind or None
 
 
 def _check(rc: int):

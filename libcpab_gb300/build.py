@@ -1,5 +1,10 @@
 """Build the sm_103a shared library libcpab_gb300/libcpab_gb300.so and the
-torch extension libcpab_gb300/_torch_bind.so over it.
+torch extension over it (_torch_bind: native autograd nodes).
+
+The extension is bound to the torch and Python that it was compiled against, and
+its file name carries both (bind_path): another torch finds no extension, never a
+foreign one, and the next build makes its own.  Without torch the C ABI library is
+built alone.
 
 Each translation unit in csrc/ is compiled by nvcc in parallel
 (-gencode arch=compute_103a,code=sm_103a) and linked into one shared library
@@ -19,7 +24,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, 'csrc')
 BUILD = os.path.join(HERE, '_build')
 LIB = os.path.join(HERE, 'libcpab_gb300.so')
-BIND = os.path.join(HERE, '_torch_bind.so')
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 
 
@@ -42,6 +46,22 @@ def _compile(nvcc, src, obj, verbose):
     return r.stderr
 
 
+def bind_path():
+    """File of the torch extension for the running Python and its torch."""
+    import sysconfig
+    import torch
+    return os.path.join(HERE, '_torch_bind-torch%s-abi%d%s'
+                        % (torch.__version__, int(torch._C._GLIBCXX_USE_CXX11_ABI),
+                           sysconfig.get_config_var('EXT_SUFFIX')))
+
+
+def _fresh(target, deps):
+    if not os.path.exists(target):
+        return False
+    t = os.path.getmtime(target)
+    return all(os.path.getmtime(d) <= t for d in deps if os.path.exists(d))
+
+
 def _compile_bind(src, obj):
     """The native autograd nodes, against the installed torch (host code only)."""
     import sysconfig
@@ -58,10 +78,10 @@ def _compile_bind(src, obj):
         raise RuntimeError('g++ failed for %s:\n%s' % (src, r.stderr))
 
 
-def _link_bind(obj):
+def _link_bind(obj, path):
     import torch
     lib = os.path.join(os.path.dirname(torch.__file__), 'lib')
-    tmp = BIND + '.tmp%d' % os.getpid()
+    tmp = path + '.tmp%d' % os.getpid()
     # the C ABI library sits next to the extension and is found through $ORIGIN
     cmd = ['g++', '-shared', '-o', tmp, obj, '-L' + HERE, '-l:libcpab_gb300.so', '-L' + lib,
            '-ltorch_python', '-ltorch', '-ltorch_cpu', '-lc10', '-lc10_cuda',
@@ -69,39 +89,45 @@ def _link_bind(obj):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError('link failed:\n' + r.stderr)
-    os.replace(tmp, BIND)
+    os.replace(tmp, path)
 
 
 def build(force=False, verbose=False):
-    """Compile if any source is newer than the libraries; returns the .so path
-    of the C ABI."""
+    """Compile what is missing or older than its sources; returns the .so path of
+    the C ABI."""
     srcs = sorted(glob.glob(os.path.join(CSRC, '*.cu')))
     bind_src = os.path.join(CSRC, 'torch_bind.cpp')
+    header = os.path.join(os.path.dirname(HERE), 'include', 'cpab_gb300.h')
     deps = srcs + glob.glob(os.path.join(CSRC, '*.cuh')) + glob.glob(os.path.join(CSRC, '*.h')) + \
-        [bind_src, os.path.join(os.path.dirname(HERE), 'include', 'cpab_gb300.h'), __file__]
-    if not force and os.path.exists(LIB) and os.path.exists(BIND):
-        t = min(os.path.getmtime(LIB), os.path.getmtime(BIND))
-        if all(os.path.getmtime(d) <= t for d in deps if os.path.exists(d)):
-            return LIB
+        [header, __file__]
+    want_lib = force or not _fresh(LIB, deps)
+    try:
+        bind = bind_path()
+    except ImportError:
+        print('torch is not importable: building the C ABI library without the torch extension')
+        bind = None
+    want_bind = bind is not None and (force or not _fresh(bind, [bind_src, header, __file__]))
     os.makedirs(BUILD, exist_ok=True)
-    nvcc = nvcc_path()
     objs = [os.path.join(BUILD, os.path.basename(s)[:-3] + '.o') for s in srcs]
     bind_obj = os.path.join(BUILD, 'torch_bind.o')
     with concurrent.futures.ThreadPoolExecutor(max_workers=min(9, len(srcs) + 1)) as ex:
-        bind = ex.submit(_compile_bind, bind_src, bind_obj)
-        logs = list(ex.map(lambda so: _compile(nvcc, so[0], so[1], verbose), zip(srcs, objs)))
-        bind.result()
-    if verbose:
-        for s, lg in zip(srcs, logs):
-            print('==', os.path.basename(s))
-            print(lg)
-    tmp = LIB + '.tmp%d' % os.getpid()
-    cmd = [nvcc, *ARCH, '-shared', '-o', tmp, *objs, '-lcudart']
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError('link failed:\n' + r.stderr)
-    os.replace(tmp, LIB)
-    _link_bind(bind_obj)
+        made = ex.submit(_compile_bind, bind_src, bind_obj) if want_bind else None
+        if want_lib:
+            nvcc = nvcc_path()
+            logs = list(ex.map(lambda so: _compile(nvcc, so[0], so[1], verbose), zip(srcs, objs)))
+            if verbose:
+                for s, lg in zip(srcs, logs):
+                    print('==', os.path.basename(s))
+                    print(lg)
+            tmp = LIB + '.tmp%d' % os.getpid()
+            cmd = [nvcc, *ARCH, '-shared', '-o', tmp, *objs, '-lcudart']
+            r = subprocess.run(cmd, capture_output=True, text=True)
+            if r.returncode != 0:
+                raise RuntimeError('link failed:\n' + r.stderr)
+            os.replace(tmp, LIB)
+        if made is not None:
+            made.result()
+            _link_bind(bind_obj, bind)
     return LIB
 
 

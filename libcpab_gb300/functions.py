@@ -169,8 +169,9 @@ def transformer(points, theta, params):
         raise ValueError('points must have %d coordinates (got %d)' % (params.ndim, points.shape[-2]))
     if params.numeric_grad:
         return TransformGridNumeric.apply(points, theta, params)
-    if native(points, theta):
-        out = N.bind().transform_grid(
+    ext = N.bind() if native(points, theta) else None
+    if ext is not None:
+        out = ext.transform_grid(
             points, theta, params, params.nc, settings(params, theta.device),
             getattr(params, 'integration', 'fixed_step') == 'exact')
         if out is not None:
@@ -208,10 +209,10 @@ def transform_data(data, theta, params, outsize):
         grid = uniform_meshgrid(params.ndim, params.domain_min, params.domain_max, outsize,
                                 data.device)
         return interpolate(params.ndim, data, transformer(grid, theta, params), outsize)
-    if native(data, theta):
-        out = N.bind().transform_data(data, theta, params, params.nc,
-                                      settings(params, data.device),
-                                      grid_axes(params, outsize, data.device), outsize)
+    ext = N.bind() if native(data, theta) else None
+    if ext is not None:
+        out = ext.transform_data(data, theta, params, params.nc, settings(params, data.device),
+                                 grid_axes(params, outsize, data.device), outsize)
         if out is not None:
             return out
     return TransformData.apply(data, theta, params, outsize)
@@ -441,9 +442,10 @@ def transform_data_mixed(data, theta, params, outsize=None):
             raise ValueError('every image must be [C, *%dD size] with the same C' % ndim)
     sizes = [tuple(int(x) for x in im.shape[1:]) for im in data]
     lay = _mixed_layout(params, sizes, outsize, theta, data)
-    if native(theta, *data):
-        outs = N.bind().transform_mixed(data, theta, params, params.nc,
-                                        settings(params, theta.device), lay, C)
+    ext = N.bind() if native(theta, *data) else None
+    if ext is not None:
+        outs = ext.transform_mixed(data, theta, params, params.nc,
+                                   settings(params, theta.device), lay, C)
         if outs is not None:
             return outs
     packed = torch.cat([im.reshape(-1).to(torch.float32) for im in data])
