@@ -79,19 +79,48 @@ Settings parse_settings(const py::handle &t) {
 }
 
 // References to params of nodes that went away on a thread without the GIL (the
-// autograd engine's): dropped by the next call that holds it, so that the engine
-// never waits for a busy interpreter (it did, 5 us and more per backward).  Every
-// node was made by such a call, so no more pile up than there were nodes.
-std::mutex g_dropped_mu;
-std::vector<PyObject *> g_dropped;
+// autograd engine's): handed to the interpreter as a pending call, so that the
+// engine never waits for a busy one (it did, 5 us and more per backward).  Should
+// the interpreter's list of those be full, the next native call drops them; every
+// node was made by such a call, so no more pile up than there were nodes.  Both
+// objects outlive the process's last node.
+std::mutex &dropped_mu() {
+    static std::mutex *mu = new std::mutex;
+    return *mu;
+}
+std::vector<PyObject *> &dropped() {   // under dropped_mu
+    static auto *v = new std::vector<PyObject *>;
+    return *v;
+}
 
 void drop_params() {   // with the GIL
     std::vector<PyObject *> v;
     {
-        std::lock_guard<std::mutex> lock(g_dropped_mu);
-        v.swap(g_dropped);
+        std::lock_guard<std::mutex> lock(dropped_mu());
+        v.swap(dropped());
     }
     for (PyObject *p : v) Py_DECREF(p);
+}
+
+void release_params(PyObject *params) {   // with or without the GIL
+    if (!Py_IsInitialized()) return;   // the interpreter and its objects are gone
+    if (PyGILState_Check()) {
+        Py_DECREF(params);
+        return;
+    }
+    bool first;
+    {
+        std::lock_guard<std::mutex> lock(dropped_mu());
+        first = dropped().empty();
+        dropped().push_back(params);
+    }
+    if (first)
+        Py_AddPendingCall(
+            [](void *) {
+                drop_params();
+                return 0;
+            },
+            nullptr);
 }
 
 // What a node keeps beside its saved tensors.
@@ -108,9 +137,7 @@ struct Kept : torch::CustomClassHolder {
     std::vector<int64_t> sizes, out_sizes;
 
     ~Kept() override {
-        if (!params) return;
-        std::lock_guard<std::mutex> lock(g_dropped_mu);
-        g_dropped.push_back(params);
+        if (params) release_params(params);
     }
 };
 
