@@ -235,6 +235,14 @@ variable_list once(bool create_graph, const variable_list &grads, variable_list 
     return out;
 }
 
+// f() with the interpreter free for other threads: allocations may synchronise and
+// launches wait for room in the queue.  Saved-tensor hooks take the GIL themselves.
+template <typename F>
+auto without_gil(const F &f) {
+    py::gil_scoped_release free;
+    return f();
+}
+
 bool needs_graph(const Tensor &a, const Tensor &b) {
     return at::GradMode::is_enabled() && (a.requires_grad() || b.requires_grad());
 }
@@ -343,13 +351,14 @@ py::object transform_grid(const Tensor &points, const Tensor &theta, const py::h
         a.kept->points_dim = points.dim();
         if (theta.dim() != 2 || theta.device() != points.device()) throw Fallback();
         a.kept->theta_dim = theta.size(1);
-        if (!needs_graph(points, theta)) {
+        const bool graph = needs_graph(points, theta);
+        if (graph) a.kept->params = params.inc_ref().ptr();
+        return py::cast(without_gil([&] {
+            if (graph) return TransformGrid::apply(points, theta, a);
             at::AutoGradMode off(false);
             Tensor A, E;
-            return py::cast(grid_forward(a, floats(points), floats(theta), false, &A, &E));
-        }
-        a.kept->params = params.inc_ref().ptr();
-        return py::cast(TransformGrid::apply(points, theta, a));
+            return grid_forward(a, floats(points), floats(theta), false, &A, &E);
+        }));
     } catch (Fallback &) {
         return py::none();
     }
@@ -443,14 +452,14 @@ py::object transform_data(const Tensor &data, const Tensor &theta, const py::han
             if (o < 1 || o > INT_MAX) throw Fallback();
         for (int64_t o : data.sizes())
             if (o > INT_MAX) throw Fallback();
-        if (!needs_graph(data, theta)) {
+        const bool graph = needs_graph(data, theta);
+        if (graph) a.kept->params = params.inc_ref().ptr();
+        return py::cast(without_gil([&] {
+            if (graph) return TransformData::apply(data, theta, a, Image{lin, {}});
             at::AutoGradMode off(false);
             Tensor A, E, grid;
-            return py::cast(
-                image_forward(a, lin, floats(data), floats(theta), false, &A, &E, &grid));
-        }
-        a.kept->params = params.inc_ref().ptr();
-        return py::cast(TransformData::apply(data, theta, a, Image{lin, {}}));
+            return image_forward(a, lin, floats(data), floats(theta), false, &A, &E, &grid);
+        }));
     } catch (Fallback &) {
         return py::none();
     }
@@ -588,7 +597,8 @@ py::object transform_mixed(const std::vector<Tensor> &images, const Tensor &thet
             k.out_sizes.push_back(C * npoints[i]);
         }
         a.kept->params = params.inc_ref().ptr();
-        return py::cast(TransformMixed::apply(at::TensorList(images), theta, a, lay));
+        return py::cast(without_gil(
+            [&] { return TransformMixed::apply(at::TensorList(images), theta, a, lay); }));
     } catch (Fallback &) {
         return py::none();
     }
