@@ -874,7 +874,7 @@ __device__ __forceinline__ bool stage_table(float *dst, const float *src, int fl
 // ---------------------------- affine helpers ---------------------------------
 // y = M[:, :N] x + M[:, N] for one cell map (row-major N x (N+1)).
 template <int N>
-__device__ __forceinline__ void affine_apply(const float *M, const float (&x)[N], float (&y)[N]) {
+CPAB_HD inline void affine_apply(const float *M, const float (&x)[N], float (&y)[N]) {
 #pragma unroll
     for (int r = 0; r < N; ++r) {
         float acc = M[r * (N + 1) + N];
