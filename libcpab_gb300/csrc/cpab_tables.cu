@@ -21,8 +21,9 @@
 // exponential.  (One thread per (theta, cell) for all of it read the basis with a
 // stride of P d between lanes, and waited on the queue of the load unit for nine
 // cycles in ten.)  64 thetas, [8,8], d = 234: 95 -> 12 us (54 us with one theta per
-// block and no chunk in flight); 4,096 thetas, [100]: 104 -> 24 us; the smallest
-// calls 7 to 9 -> 4 to 5 us.
+// block and no chunk in flight); 4,096 thetas, [100]: 104 -> 24 us; 16 thetas of
+// [50], d = 50, back to back 4.4 -> 3.2 us.  Small bases keep the one thread
+// (k_cell_tables_small).
 #include "cpab_expm.cuh"
 
 namespace cpab {
@@ -32,6 +33,31 @@ template <int N>
 __host__ __device__ constexpr int tile_cells() { return N == 1 ? 64 : N == 2 ? 32 : 16; }
 template <int N>
 __host__ __device__ constexpr int tile_rows() { return tile_cells<N>() * N * (N + 1); }
+
+// T = expm(dt [A;0]) and E = T - I (either may be null) of one cell, from its rows a
+// of A, to element off.
+template <int N>
+__device__ __forceinline__ void store_exp(const float *a, float dt, long long off,
+                                          float *__restrict__ T, float *__restrict__ E) {
+    float M[N][N], v[N], El[N][N], Et[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) M[r][j] = a[r * (N + 1) + j] * dt;
+        v[r] = a[r * (N + 1) + N] * dt;
+    }
+    expm1_affine<N>(M, v, El, Et);
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            if (E) E[off + r * (N + 1) + j] = El[r][j];
+            if (T) T[off + r * (N + 1) + j] = El[r][j] + ((r == j) ? 1.f : 0.f);
+        }
+        if (E) E[off + r * (N + 1) + N] = Et[r];
+        if (T) T[off + r * (N + 1) + N] = Et[r];
+    }
+}
 
 template <int N, int TB>
 __global__ void __launch_bounds__(tile_rows<N>())
@@ -96,27 +122,53 @@ __global__ void __launch_bounds__(tile_rows<N>())
     __syncthreads();
     for (int i = tid; i < nt * nc; i += R) {
         const int q = i / nc, c = i - q * nc;
-        const float *a = a_s + q * R + c * P;
-        const long long off = ((long long)(th0 + q) * nC + c0 + c) * P;
-        float M[N][N], v[N], El[N][N], Et[N];
-#pragma unroll
-        for (int r = 0; r < N; ++r) {
-#pragma unroll
-            for (int j = 0; j < N; ++j) M[r][j] = a[r * (N + 1) + j] * dt;
-            v[r] = a[r * (N + 1) + N] * dt;
-        }
-        expm1_affine<N>(M, v, El, Et);
-#pragma unroll
-        for (int r = 0; r < N; ++r) {
-#pragma unroll
-            for (int j = 0; j < N; ++j) {
-                if (E) E[off + r * (N + 1) + j] = El[r][j];
-                if (T) T[off + r * (N + 1) + j] = El[r][j] + ((r == j) ? 1.f : 0.f);
-            }
-            if (E) E[off + r * (N + 1) + N] = Et[r];
-            if (T) T[off + r * (N + 1) + N] = Et[r];
-        }
+        store_exp<N>(a_s + q * R + c * P, dt, ((long long)(th0 + q) * nC + c0 + c) * P, T, E);
     }
+}
+
+// Small bases (see small_basis): one thread per (theta, cell) does all of it.  The
+// basis stays in L1, and no lane waits for a tile to fill: 100,000 thetas of [2],
+// d = 1, 6 us against 55 us on tiles, 65,536 of [20], d = 10, 16 against 41 us, 16 of
+// [10], d = 5, 1.7 against 2.2 us.
+template <int N>
+__global__ void __launch_bounds__(128)
+    k_cell_tables_small(int nC, float dt, const float *__restrict__ theta, int n_theta, int d,
+                        const float *__restrict__ basis, float *__restrict__ A,
+                        float *__restrict__ T, float *__restrict__ E) {
+    constexpr int P = N * (N + 1);
+    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid >= (long long)n_theta * nC) return;
+    const long long th = gid / nC;
+    const float *tv = theta + th * d, *rows = basis + (gid - th * nC) * P * d;
+    float a[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) a[i] = 0.f;
+    for (int k = 0; k < d; ++k) {
+        const float tk = __ldg(tv + k);
+#pragma unroll
+        for (int i = 0; i < P; ++i) a[i] = fmaf(__ldg(rows + i * d + k), tk, a[i]);
+    }
+    if (A) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) A[gid * P + i] = a[i];
+    }
+    if (T || E) store_exp<N>(a, dt, gid * P, T, E);
+}
+
+// Where one thread per (theta, cell) is the faster way, from both ways measured over
+// [1] .. [16,16] and [4,4,4], d from a tenth to half of the rows, 1 to 500,000 thetas:
+// 4 KB of basis or less, with up to 50 loads per thread (from there on its chain of
+// loads is longer than the tile's barriers: [2,2], d = 9, 54 loads, equal; [20], d =
+// 20, 40 loads, equal) or with thousands of thetas, which hide the chain ([1,1],
+// d = 12, 65,536 thetas 8 against 103 us, 1,024 thetas 2.4 against 2.8 us).  With those also
+// 8 KB, where the cells fill a third of a tile at most ([1,1,1], d = 30: 43 against
+// 127 us).  Above, tiles: [50], d = 25, 65,536 thetas 60 us against 180 us.
+template <int N>
+static bool small_basis(int nC, int d, int n_theta) {
+    constexpr int P = N * (N + 1);
+    const long long floats = (long long)nC * P * d;
+    if (floats <= 1024) return P * d <= 50 || n_theta >= 4096;
+    return floats <= 2048 && n_theta >= 4096 && 3 * nC <= tile_cells<N>();
 }
 
 // Eight or four thetas per block (the basis is then read once for them) as long
@@ -126,6 +178,13 @@ template <int N>
 static cudaError_t launch_tables(int nC, float dt, const float *theta, int n_theta, int d,
                                  const float *basis, float *A, float *T, float *E,
                                  cudaStream_t s) {
+    if (small_basis<N>(nC, d, n_theta)) {
+        const long long grid = ((long long)n_theta * nC + 127) / 128;
+        if (grid >= (1ll << 31)) return cudaErrorInvalidConfiguration;
+        k_cell_tables_small<N><<<(unsigned)grid, 128, 0, s>>>(nC, dt, theta, n_theta, d, basis, A,
+                                                              T, E);
+        return cudaGetLastError();
+    }
     int tiles = (nC + tile_cells<N>() - 1) / tile_cells<N>(), tb = 8;
     auto blocks = [&] { return (n_theta + tb - 1ll) / tb * tiles; };
     if (2 * blocks() < num_sms()) tb = 4;
