@@ -389,10 +389,11 @@ __global__ void __launch_bounds__(256, tma_blocks_per_sm<N, CC>())
 // neighbouring pixels, so sums that meet go out as one: where the next lane's
 // low corners on the last axis are this lane's high ones, and where the next
 // row's (x + 1) low-x corners are this row's high-x ones, which a warp that
-// takes four consecutive x holds back for it.  256 x 3 x 224^2, a smooth warp:
-// 0.351 ms channel by channel, 0.298 ms with the loads ahead, 0.280 ms with the
-// lanes' sums shared, 0.228 ms with the rows' too.
-// CC = 0: any C, channel by channel.
+// takes consecutive x holds back for it (the rows of a tile that the image's edge
+// cuts are spread over all warps: 4 x 8 x 40^3 would leave six of eight idle in a
+// fifth of the tiles).  256 x 3 x 224^2, a smooth warp: 0.351 ms channel by channel,
+// 0.298 ms with the loads ahead, 0.280 ms with the lanes' sums shared, 0.228 ms with
+// the rows' too.
 // Offset of the corner with bits m on the axes after x.
 template <int N>
 __device__ __forceinline__ int high_delta(const int (&step)[N], int m) {
@@ -422,15 +423,16 @@ __global__ void __launch_bounds__(256, backward_blocks<N, CC>())
         __syncthreads();
         load_grid_tile<N>(g, grid + (long long)b * N * g.nP, a0, z0, mid, sp);
         __syncthreads();
-        constexpr int H = 1 << (N - 1), RR = kTile / kRows;
-        // sums of a row's high-x corners, held back for the next row (CC > 0)
-        float pend[CC > 0 ? CC : 1][H];
+        constexpr int H = 1 << (N - 1);
+        const int per = (min(A - a0, kTile) + kRows - 1) / kRows;
+        // sums of a row's high-x corners, held back for the next row
+        float pend[CC][H];
         int pbase = -1, pstep[N];   // element of the first of them (-1: none)
         bool pgive = false;
 #pragma unroll 1
-        for (int r = 0; r < RR; ++r) {
-            // a warp takes RR consecutive x
-            const int al = ty * RR + r, a = a0 + al, z = z0 + tx;
+        for (int r = 0; r < per; ++r) {
+            // a warp takes consecutive x
+            const int al = ty * per + r, a = a0 + al, z = z0 + tx;
             if (a >= A) break;   // the whole warp
             const bool live = z < Z;
             float p[N], gf[N];
@@ -440,88 +442,136 @@ __global__ void __launch_bounds__(256, backward_blocks<N, CC>())
                 gf[j] = 0.f;
             }
             const int o = out_index<N>(g, a, mid, live ? z : z0);
-            if constexpr (CC > 0) {
-                const CornerStep<N> cr = corner_steps<N, false>(p, g);
-                const long long plane = (long long)b * CC;
-                const float *D = data + plane * g.nD + cr.base;
-                float v[CC][1 << N], w[CC];
+            const CornerStep<N> cr = corner_steps<N, false>(p, g);
+            const long long plane = (long long)b * CC;
+            const float *D = data + plane * g.nD + cr.base;
+            float v[CC][1 << N], w[CC];
 #pragma unroll
-                for (int c = 0; c < CC; ++c) {
-                    w[c] = __ldg(gout + (plane + c) * g.nP + o);
+            for (int c = 0; c < CC; ++c) {
+                w[c] = __ldg(gout + (plane + c) * g.nP + o);
 #pragma unroll
-                    for (int m = 0; m < (1 << N); ++m)
-                        v[c][m] = __ldg(D + (long long)c * g.nD + cr.delta(m));
+                for (int m = 0; m < (1 << N); ++m)
+                    v[c][m] = __ldg(D + (long long)c * g.nD + cr.delta(m));
+            }
+            // this row's low-x corners are the last row's high-x ones
+            bool same = live && pbase == cr.base;
+            // the next lane's low corners on the last axis are this lane's high ones
+            const int next = __shfl_down_sync(0xffffffffu, live ? cr.base : -1, 1);
+            bool give = live && tx < 31 && cr.step[N - 1] != 0 && next == cr.base + 1;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                if (j > 0) same &= pstep[j] == cr.step[j];
+                if (j < N - 1) give &= __shfl_down_sync(0xffffffffu, cr.step[j], 1) == cr.step[j];
+            }
+            const bool take = __shfl_up_sync(0xffffffffu, give, 1) && tx > 0;
+            const bool old = pbase >= 0 && !same;
+#pragma unroll
+            for (int c = 0; c < CC; ++c) {
+                float wt[1 << N];
+                lerp_grads_of<N>(v[c], cr.f, w[c], gf, [&](int m, float x) { wt[m] = x; });
+                if (!ddata) continue;
+                float *Sc = ddata + (plane + c) * g.nD;
+#pragma unroll
+                for (int m = 0; m < H; ++m) {   // m: corner bits of the axes after x
+                    if (old) atomicAdd(Sc + pbase + high_delta<N>(pstep, m), pend[c][m]);
+                    if (same) wt[2 * m] += pend[c][m];
+                    pend[c][m] = wt[2 * m + 1];
                 }
-                // this row's low-x corners are the last row's high-x ones
-                bool same = live && pbase == cr.base;
-                // the next lane's low corners on the last axis are this lane's high ones
-                const int next = __shfl_down_sync(0xffffffffu, live ? cr.base : -1, 1);
-                bool give = live && tx < 31 && cr.step[N - 1] != 0 && next == cr.base + 1;
 #pragma unroll
-                for (int j = 0; j < N; ++j) {
-                    if (j > 0) same &= pstep[j] == cr.step[j];
-                    if (j < N - 1) give &= __shfl_down_sync(0xffffffffu, cr.step[j], 1) == cr.step[j];
-                }
-                const bool take = __shfl_up_sync(0xffffffffu, give, 1) && tx > 0;
-                const bool old = pbase >= 0 && !same;
-#pragma unroll
-                for (int c = 0; c < CC; ++c) {
-                    float wt[1 << N];
-                    lerp_grads_of<N>(v[c], cr.f, w[c], gf, [&](int m, float x) { wt[m] = x; });
-                    if (!ddata) continue;
-                    float *Sc = ddata + (plane + c) * g.nD;
-#pragma unroll
-                    for (int m = 0; m < H; ++m) {   // m: corner bits of the axes after x
-                        if (old) atomicAdd(Sc + pbase + high_delta<N>(pstep, m), pend[c][m]);
-                        if (same) wt[2 * m] += pend[c][m];
-                        pend[c][m] = wt[2 * m + 1];
+                for (int m = 0; m < H / 2; ++m) {
+                    const int lo = 2 * m, hi = 2 * (m | (H / 2));
+                    const float from = __shfl_up_sync(0xffffffffu, wt[hi], 1);
+                    if (live) {
+                        atomicAdd(Sc + cr.base + cr.delta(lo), take ? wt[lo] + from : wt[lo]);
+                        if (!give) atomicAdd(Sc + cr.base + cr.delta(hi), wt[hi]);
                     }
-#pragma unroll
-                    for (int m = 0; m < H / 2; ++m) {
-                        const int lo = 2 * m, hi = 2 * (m | (H / 2));
-                        const float from = __shfl_up_sync(0xffffffffu, wt[hi], 1);
-                        if (live) {
-                            atomicAdd(Sc + cr.base + cr.delta(lo), take ? wt[lo] + from : wt[lo]);
-                            if (!give) atomicAdd(Sc + cr.base + cr.delta(hi), wt[hi]);
-                        }
-                    }
-                }
-                pbase = live ? cr.base + cr.step[0] : -1;
-                pgive = give;
-#pragma unroll
-                for (int j = 0; j < N; ++j) pstep[j] = cr.step[j];
-                if (!live) continue;
-            } else {
-                if (!live) continue;
-                const Corner<N> cr = corners<N>(p, g);
-                for (int c = 0; c < C; ++c) {
-                    const long long plane = (long long)b * C + c;
-                    const float w = __ldg(gout + plane * g.nP + o);
-                    lerp_grads<N>(data + plane * g.nD, cr, w,
-                                  ddata ? ddata + plane * g.nD : nullptr, gf);
                 }
             }
+            pbase = live ? cr.base + cr.step[0] : -1;
+            pgive = give;
+#pragma unroll
+            for (int j = 0; j < N; ++j) pstep[j] = cr.step[j];
+            if (!live) continue;
 #pragma unroll
             for (int j = 0; j < N; ++j) sp[j][tx][al] = gf[j] * g.sizem1[j];
         }
-        if constexpr (CC > 0) {
-            if (ddata) {
-                const bool live = pbase >= 0;
-                const bool take = __shfl_up_sync(0xffffffffu, pgive, 1) && tx > 0;
+        if (ddata) {
+            const bool live = pbase >= 0;
+            const bool take = __shfl_up_sync(0xffffffffu, pgive, 1) && tx > 0;
 #pragma unroll
-                for (int c = 0; c < CC; ++c) {
-                    float *Sc = ddata + ((long long)b * CC + c) * g.nD + pbase;
+            for (int c = 0; c < CC; ++c) {
+                float *Sc = ddata + ((long long)b * CC + c) * g.nD + pbase;
 #pragma unroll
-                    for (int m = 0; m < H / 2; ++m) {
-                        const float from = __shfl_up_sync(0xffffffffu, pend[c][m | (H / 2)], 1);
-                        if (live) {
-                            atomicAdd(Sc + high_delta<N>(pstep, m), take ? pend[c][m] + from : pend[c][m]);
-                            if (!pgive)
-                                atomicAdd(Sc + high_delta<N>(pstep, m | (H / 2)), pend[c][m | (H / 2)]);
-                        }
+                for (int m = 0; m < H / 2; ++m) {
+                    const float from = __shfl_up_sync(0xffffffffu, pend[c][m | (H / 2)], 1);
+                    if (live) {
+                        atomicAdd(Sc + high_delta<N>(pstep, m), take ? pend[c][m] + from : pend[c][m]);
+                        if (!pgive)
+                            atomicAdd(Sc + high_delta<N>(pstep, m | (H / 2)), pend[c][m | (H / 2)]);
                     }
                 }
             }
+        }
+        if (!dgrid) continue;
+        __syncthreads();
+        float *db = dgrid + (long long)b * N * g.nP;
+#pragma unroll
+        for (int r = 0; r < kTile / kRows; ++r) {
+            const int zl = ty + kRows * r, a = a0 + tx, z = z0 + zl;
+            if (a < A && z < Z) {
+                const int k = grid_index<N>(g, a, mid, z);
+#pragma unroll
+                for (int j = 0; j < N; ++j) db[(long long)j * g.nP + k] = sp[j][zl][tx];
+            }
+        }
+    }
+}
+
+// Any C, channel by channel: no sum waits for a neighbour, and a row's corners come
+// from L1 where the row before read them.  A kernel of its own: as a branch of the one
+// above it was slower the more channels there were (64 x 16 x 160^2 0.254 ms, 0.205 now
+// and 0.231 with the rows unrolled and a warp's rows apart; 5 channels 0.084, 0.073 and
+// 0.083).  BLOCKS per SM: in 3D two, where the last wave is shorter and the gathers
+// evict each other less (2 x 8 x 32 x 96^2 0.070 ms, 0.091 with three; 8 x 3 x 64^3
+// 0.097 and 0.101; an uncorrelated grid, 8 x 8 x 40^3, 0.255 and 0.274; magnified
+// images, which L1 serves, lose: 8 x 3 x 64^3 0.127 and 0.119).
+template <int N, int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS)
+    k_interpolate_backward_channels(Geo g, TileGeo tg, const float *__restrict__ data, int C,
+                                    const float *__restrict__ grid,
+                                    const float *__restrict__ gout, float *__restrict__ ddata,
+                                    float *__restrict__ dgrid, int nb) {
+    __shared__ float sp[N][kTile][kTile + 1];
+    int a0, z0, mid;
+    tile_coords<N>(g, tg, blockIdx.x, a0, z0, mid);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int A = g.outsize[0], Z = g.outsize[N - 1];
+    for (int b = blockIdx.y; b < nb; b += gridDim.y) {
+        __syncthreads();
+        load_grid_tile<N>(g, grid + (long long)b * N * g.nP, a0, z0, mid, sp);
+        __syncthreads();
+        const int per = (min(A - a0, kTile) + kRows - 1) / kRows;
+#pragma unroll 1
+        for (int r = 0; r < per; ++r) {
+            const int al = ty * per + r;
+            const int a = a0 + al, z = z0 + tx;
+            if (a >= A || z >= Z) continue;
+            float p[N], gf[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                p[j] = sp[j][tx][al];
+                gf[j] = 0.f;
+            }
+            const Corner<N> cr = corners<N>(p, g);
+            const int o = out_index<N>(g, a, mid, z);
+            for (int c = 0; c < C; ++c) {
+                const long long plane = (long long)b * C + c;
+                const float w = __ldg(gout + plane * g.nP + o);
+                lerp_grads<N>(data + plane * g.nD, cr, w, ddata ? ddata + plane * g.nD : nullptr,
+                              gf);
+            }
+#pragma unroll
+            for (int j = 0; j < N; ++j) sp[j][tx][al] = gf[j] * g.sizem1[j];
         }
         if (!dgrid) continue;
         __syncthreads();
@@ -672,6 +722,9 @@ cudaError_t launch_interpolate_backward(int ndim, const float *data, int nb, int
     unsigned blocks = 0;
     const TileGeo tg = make_tiles(ndim, g, &blocks);
     const dim3 tgrid(blocks, gridn.y);
+#define CPAB_IBC(NN, BLOCKS)                                                                   \
+    k_interpolate_backward_channels<NN, BLOCKS><<<tgrid, block, 0, s>>>(g, tg, data, C, grid, \
+                                                                        gout, ddata, dgrid, nb)
 #define CPAB_IB(NN, CC)                                                                        \
     k_interpolate_backward_tiled<NN, CC><<<tgrid, block, 0, s>>>(g, tg, data, C, grid, gout,  \
                                                                  ddata, dgrid, nb)
@@ -681,16 +734,17 @@ cudaError_t launch_interpolate_backward(int ndim, const float *data, int nb, int
             case 2: CPAB_IB(2, 2); break;
             case 3: CPAB_IB(2, 3); break;
             case 4: CPAB_IB(2, 4); break;
-            default: CPAB_IB(2, 0); break;
+            default: CPAB_IBC(2, 3); break;
         }
     } else {
         switch (C) {
             case 1: CPAB_IB(3, 1); break;
             case 2: CPAB_IB(3, 2); break;
-            default: CPAB_IB(3, 0); break;
+            default: CPAB_IBC(3, 2); break;
         }
     }
 #undef CPAB_IB
+#undef CPAB_IBC
     return cudaGetLastError();
 }
 
