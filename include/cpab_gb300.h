@@ -257,8 +257,9 @@ CPAB_API int cpab_integrate_exact(int ndim, const int *nc, const float *points, 
  * [n_theta, ndim, nP] is cpab_integrate_exact's result for the same A.  The
  * flow is integrated backwards from out in certified in-cell sub-steps; per
  * sub-step the cotangent is carried back through the in-cell flow and dL/dA
- * gathers the adjoint Frechet derivative of its exponential.  The field is
- * continuous across faces, so the crossing times add no term.  workspace:
+ * gathers the integral of cotangent times point along it (Gauss-Legendre
+ * quadrature).  The field is continuous across faces, so the crossing times add
+ * no term.  workspace:
  * cpab_backward_exact_workspace() bytes of device memory.
  */
 CPAB_API size_t cpab_backward_exact_workspace(int ndim, const int *nc, long long nP,

@@ -45,11 +45,12 @@
 // same cell at the same step are first summed in lane order (match.any and
 // shuffles), so each table element receives at most one add per step, in
 // step order.  At the end the warp copies are summed in warp order into one
-// partial per CTA, and k_finalize sums the partials in CTA order.  No
-// floating-point atomics are used, so the result is bit-reproducible for a
-// given GPU and input.  In 1D, where the lanes of a sorted grid sit in
-// non-decreasing cells, the lane groups are found without match.any
-// (warp_flush_1d).  For large tessellations the per-warp tables live in the
+// partial per CTA, and k_finalize sums the partials in a fixed order.  Where the
+// tables are in global memory an addition is an atomic reduction, but no two are
+// ever in a race: an element gets one per flush, and __syncwarp orders the flushes.
+// So the result is bit-reproducible for a given GPU and input.  In 1D, where the
+// lanes of a sorted grid sit in non-decreasing cells, the lane groups are found
+// without match.any (warp_flush_1d).  For large tessellations the per-warp tables live in the
 // workspace instead of shared memory when that fits more warps per SM
 // (adjoint_shape, carve_adjoint).
 #include "cpab_adjoint.cuh"

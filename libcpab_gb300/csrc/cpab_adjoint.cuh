@@ -311,10 +311,11 @@ struct AdjSmem {
     CT *cl;
 };
 
-// GWG: gw_ext is this CTA's W per-warp tables in global memory (L2-resident;
-// each warp owns its table, so the flush stays a plain read-add-write), else
-// the tables are in shared memory.  Global tables free shared memory for more
-// resident warps when the tables are large (3D, hundreds of cells).
+// GWG: gw_ext is this CTA's W per-warp tables in global memory (L2-resident; each
+// warp owns its table and adds to it by reductions, see table_add), else the tables
+// are in shared memory and the flush is a read, an addition and a write.  Global
+// tables free shared memory for more resident warps when the tables are large (3D,
+// hundreds of cells).
 template <int N, typename CT, bool GWG = false>
 __device__ __forceinline__ AdjSmem<N, CT> carve_adjoint(float *base, int nC, int nsteps,
                                                         float *gw_ext = nullptr) {

@@ -4,18 +4,21 @@
 // -----------
 // The reference decides the cell of a point in double precision
 // (libcpab/core/cpab_ops.cu:21-227 for CUDA, libcpab/core/cpab_ops.cpp:26-184
-// for the CPU).  GB300 has a low FP64 rate, so lookups here run in FP32:
-//   * the cell index along each axis (floor(p/inc)) and the remainder
-//     p - i*inc are computed exactly with two FMAs (split_exact);
-//   * the sub-cell tests (triangle diagonals, tetrahedron planes; in 2D also
-//     the out-of-domain rules, which are the same tests on the edge square)
-//     use FP32 values with a proven error bound; when a test lands within its
-//     margin of zero, the lookup is redone with an FP64 replica of the
-//     reference's arithmetic.
+// for the CPU).  GB300 has a low FP64 rate, so lookups here run in FP32, in tiers:
+//   * the first decides nearly every point with a few products: in 2D square and
+//     triangle wherever each is clear of a margin that covers their rounding
+//     (cell_2d_quick), in 3D with power-of-two cell counts the exact cube and the
+//     tetrahedron with a margin (cell_3d_quick);
+//   * the next computes the index along each axis (floor(p/inc)) and the remainder
+//     p - i*inc exactly with two FMAs (split_exact) and decides what that leaves
+//     open: with FP32 pairs where the cells are square (cell_2d_tier2) or the counts
+//     powers of two (cell_3d_tier2), else with a margin (cell_2d_fast,
+//     cell_3d_fast);
+//   * the last is an FP64 replica of the reference's arithmetic.
 // The result is bit-identical to the reference lookup for every float input.
-// The FP64 branch is taken only for genuine near-ties (a point within ~2e-6 of
-// a diagonal or plane, including 3D points pushed onto a domain corner) and
-// non-finite input; it is counted when a counter is supplied.
+// The FP64 branch is taken only for genuine near-ties (where no tier above is
+// exact, a point within ~2e-6 of a diagonal or plane) and non-finite input; it is
+// counted when a counter is supplied.
 //
 // Tables
 // ------

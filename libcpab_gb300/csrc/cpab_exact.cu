@@ -19,10 +19,10 @@
 //     most |v(p)| + ||A_lin|| (d + e), so a step of time (d + e) / that bound
 //     stays in the cell or passes a face by at most e = 1e-5 (where the two
 //     cells' fields differ by O(e)).  Each step uses the exact in-cell flow,
-//     p + sum_k dt^k A_lin^(k-1) v / k! (|A| dt < 1 by the rule; the series on
-//     the vector takes 60 operations where the matrix E(dt) took 180); the cell
-//     is looked up with the reference's rules before each step.  Steps shrink
-//     geometrically towards a face, so a crossing costs ~10-20 steps; a
+//     p + sum_k dt^k A_lin^(k-1) v / k! (|A| dt <= 1 by the rule; the series on
+//     the vector takes 60 operations where the matrix E(dt) took 180; cpab_flow.cuh);
+//     the cell is looked up with the reference's rules before each step.  Steps
+//     shrink geometrically towards a face, so a crossing costs ~10-20 steps; a
 //     trajectory that needs more than kExactMaxIter steps raises kErrIterLimit
 //     and returns its position at that point.
 #include "cpab_adjoint.cuh"

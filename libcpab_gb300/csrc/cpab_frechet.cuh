@@ -1,5 +1,5 @@
-// Frechet derivative of the matrix exponential, shared by the finalize kernel
-// (cpab_finalize.cu) and the exact-flow adjoint (cpab_exact.cu).
+// Frechet derivative of the matrix exponential, for the finalize kernel
+// (cpab_finalize.cu).
 #pragma once
 #include "cpab_launch.h"
 
@@ -9,10 +9,9 @@ namespace cpab {
 // recursion on Y/2^s, E/2^s followed by s squarings:
 //   R_{k-1} = I + (Y/k) R_k,  dR_{k-1} = (E/k) R_k + (Y/k) dR_k,
 //   then  L <- L R + R L,  R <- R R.
-// Rout receives R = expm(Y) (the overload without it drops R).
 template <int K>
 __device__ __forceinline__ void frechet_expm(const float (&Y0)[K][K], const float (&E0)[K][K],
-                                             float (&L)[K][K], float (&Rout)[K][K]) {
+                                             float (&L)[K][K]) {
     float norm = 0.f;
 #pragma unroll
     for (int j = 0; j < K; ++j) {
@@ -79,17 +78,6 @@ __device__ __forceinline__ void frechet_expm(const float (&Y0)[K][K], const floa
     for (int i = 0; i < K; ++i)
 #pragma unroll
         for (int j = 0; j < K; ++j) L[i][j] = D[i][j];
-#pragma unroll
-    for (int i = 0; i < K; ++i)
-#pragma unroll
-        for (int j = 0; j < K; ++j) Rout[i][j] = R[i][j];
-}
-
-template <int K>
-__device__ __forceinline__ void frechet_expm(const float (&Y0)[K][K], const float (&E0)[K][K],
-                                             float (&L)[K][K]) {
-    float R[K][K];
-    frechet_expm<K>(Y0, E0, L, R);
 }
 
 }  // namespace cpab

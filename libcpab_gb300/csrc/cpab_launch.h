@@ -113,9 +113,10 @@ constexpr int kFinalizeDirect = 3;
 cudaError_t launch_finalize(const Tess &t, int nsteps, int mode, const float *partials, int parts,
                             const float *A, const float *basis, int d, int n_theta,
                             float *dtheta, cudaStream_t s);
-// The same for ragged sets, whose partials are the slots w + s of the `warps`
-// warps of the adjoint launch (cpab_ragged.cuh); sse_partials / sse (may be
-// null): per-series squared error of the fused 1D MSE; dtheta may be null.
+// The same for ragged sets, whose partials are the slots v + s of the `chunks`
+// chunks of the adjoint launch, which `warps` warps took up (tile_chunks,
+// cpab_ragged.cuh); sse_partials / sse (may be null): per-series squared error of
+// the fused 1D MSE; dtheta may be null.
 cudaError_t launch_ragged_finalize(const Tess &t, int nsteps, int mode, const float *partials,
                                    const int *tile_off, int S, int warps, int chunks,
                                    const float *A,
@@ -259,9 +260,9 @@ struct RaggedBwd {
     float loss_scale;      // fused MSE: dL/d(out) = loss_scale * (out - target)
     float *out;            // [total] (fused MSE, optional)
     float *dvalues;        // [total] (optional, accumulated)
-    float *partials;       // [(TW + S)][nC * 2]  (set from the workspace)
-    float *sse_partials;   // [(TW + S)]          (set from the workspace)
-    float *lane_slots;     // [TW][nC][32][2] per-lane cell sums, nC <= kLaneSlotCells
+    float *partials;       // [(chunks + S)][nC * 2]  (set from the workspace)
+    float *sse_partials;   // [(chunks + S)]          (set from the workspace)
+    float *lane_slots;     // [warps][nC][32][2] per-lane cell sums, nC <= kLaneSlotCells
                            // (set from the workspace)
 };
 // fused = true: dL/d(out) from the MSE residual against `target`, per-series

@@ -12,20 +12,21 @@
 //     tile prefix over series (tile_off, S + 1 ints) is built on the device by
 //     k_ragged_plan, so nothing waits for the host and the whole sequence can
 //     be captured in a CUDA graph;
-//   * each warp owns a contiguous range of K = ceil(tiles / warps) tiles; it
-//     finds its first series by binary search in tile_off and walks forward,
-//     restaging the series' cell table into its own slice of shared memory
-//     when the series changes;
+//   * the forward gives each warp a contiguous range of K = ceil(tiles / warps)
+//     tiles, the adjoint cuts the tiles into contiguous chunks and hands them out as
+//     warps get done (tile_chunks, cpab_ragged.cuh); a warp finds the first series
+//     of its range by binary search in tile_off and walks forward, restaging the
+//     series' cell table into its own slice of shared memory when the series changes;
 //   * a series' grid is monotone, so the lanes of a warp tile are already
 //     bucketed by starting cell (neighbouring lanes start in the same or the
 //     next cell) and no sort is needed;
 //   * dtheta: a warp accumulates its series' cell statistics in its own table
-//     (warp flush of cpab_adjoint.cuh) and, when it leaves the series, writes
-//     them to partial slot (warp + series).  Warps own contiguous tile ranges,
-//     so series s is touched exactly by warps tile_off[s]/K ..
-//     (tile_off[s+1]-1)/K and the slots of all touched (warp, series) pairs
-//     are distinct.  k_finalize sums a series' slots in warp order:
-//     deterministic, no atomics.
+//     (warp flush of cpab_adjoint.cuh, or per-lane slots) and, when it leaves the
+//     series or the chunk ends, writes them to partial slot (chunk + series).
+//     Chunks are contiguous tile ranges, so series s is touched exactly by the chunks
+//     of its tiles and the slots of all touched (chunk, series) pairs are distinct,
+//     whichever warps ran them.  k_finalize sums a series' slots in chunk order:
+//     deterministic.
 //
 // The trajectory arithmetic is that of the other kernels: compensated update
 // p <- p + E [p;1] for the transformed grid (bit-identical to cpab_integrate
@@ -473,7 +474,8 @@ static cudaError_t launch_ra_ls(const Tess &t, int nsteps, int block, int ppt, i
     const int warps = grid * (block / 32), chunks = num_sms() * kChunksPerSM;
     kern<<<grid, block, smem, s>>>(t, nsteps, st, S, off, tile_off, chunks, ppt, a, ties, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    return launch_ragged_finalize(t, nsteps, MODE, a.partials, tile_off, S, warps, chunks, a.A, basis, d, dtheta, a.sse_partials, sse, s);
+    return launch_ragged_finalize(t, nsteps, MODE, a.partials, tile_off, S, warps, chunks, a.A,
+                                  basis, d, dtheta, a.sse_partials, sse, s);
 }
 
 template <int MODE, typename CT, bool FUSED>

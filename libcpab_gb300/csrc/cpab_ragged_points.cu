@@ -7,7 +7,7 @@
 //
 // Same structure as the 1D series kernels (cpab_ragged.cuh): warp tiles of one
 // set, the set's tables restaged into the warp's own shared-memory slice when
-// the set changes, per-(warp, set) partial slots for a deterministic dtheta.
+// the set changes, per-(chunk, set) partial slots for a deterministic dtheta.
 // The forward integrates PPT points per lane with the compensated update of
 // k_integrate; the backward runs the trajectory adjoint of cpab_adjoint.cuh
 // (logged forward, segment rebuild, reverse sweep with warp flushes) and
