@@ -55,11 +55,16 @@ CPAB_HD inline float face_distance(const float (&p)[N], const Tess &t) {
     return fmaxf(d - 4e-7f * imin, 0.f);
 }
 
-// Root and reciprocal of a step's bound, in one instruction each on the GPU: within
-// 2^-22 of the exact ones (the rounded ones were a fifth of a step's dependent chain,
-// and a trajectory that slides along a face takes thousands of steps one after the
-// other: 64 x 224^2, forward and gradient, 3.96 ms, rounded 4.14).  On the host the
-// rounded ones, off by CPAB_FLOW_ERROR, which the test sets to the ends of that range.
+// Root and quotient of a step's bound, approximate on the GPU: within 2^-22 of the exact
+// ones (the rounded ones were a fifth of a step's dependent chain, and a trajectory
+// that slides along a face takes thousands of steps one after the other: 64 x 224^2,
+// forward and gradient, 3.96 ms, rounded 4.14).  With five roundings of 2^-24 a step
+// is at most 2^-20 longer than the exact rule's, so it passes a face by at most
+// kOvershoot + 2^-20.  (Taken off the step instead, that changes which steps a
+// trajectory takes that ends at the limit of their number, and its result with them
+// by up to 1e-3.)  The quotient is 0 for a bound above 2^126, which no finite speed
+// gives: its square has overflowed at 2^64.  On the host the rounded ones, off by
+// CPAB_FLOW_ERROR, which the test sets to the ends of the range.
 #ifndef CPAB_FLOW_ERROR
 #define CPAB_FLOW_ERROR 0.f
 #endif
@@ -72,19 +77,13 @@ CPAB_HD inline float bound_root(float x) {
     return sqrtf(x) * (1.f + CPAB_FLOW_ERROR);
 #endif
 }
-CPAB_HD inline float bound_reciprocal(float x) {
+CPAB_HD inline float bound_quotient(float a, float b) {
 #if defined(__CUDA_ARCH__)
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
+    return __fdividef(a, b);
 #else
-    return (1.f / x) * (1.f - CPAB_FLOW_ERROR);
+    return (a / b) * (1.f - CPAB_FLOW_ERROR);
 #endif
 }
-
-// Taken off a step for them: two errors of 2^-22 and five roundings of 2^-24 make
-// less than 2^-20, so that the step is never longer than the exact rule's.
-constexpr float kStepSlack = 9.5367431640625e-07f;   // 2^-20
 
 // Velocity at p in cell map M, and the certified step there; negative for a
 // field that vanishes at p and has no linear part, or NaN input.
@@ -102,7 +101,7 @@ CPAB_HD inline float certified_step(const float (&M)[N * (N + 1)], const float (
     const float reach = face_distance<N>(p, t) + kOvershoot;
     norm = bound_root(anorm2);
     const float bound = bound_root(speed2) + norm * reach;
-    return bound > 0.f ? (reach - reach * kStepSlack) * bound_reciprocal(bound) : -1.f;
+    return bound > 0.f ? bound_quotient(reach, bound) : -1.f;
 }
 
 // Terms of the in-cell flow's series: with |A| dt < 1 the first one left out is
