@@ -45,11 +45,11 @@ FLOP_FWD_STEP, FLOP_ADJ_STEP = 17, 37
 # thread instructions per point-step of the fused kernels (2D [3,3], reference
 # gradient), from the ncu capture of 16 images summarised in profiles/
 # (smsp__inst_executed x active threads per instruction / point-steps)
-INSTR_FWD_STEP, INSTR_BWD_STEP = 52, 193
+INSTR_FWD_STEP, INSTR_BWD_STEP = 53, 191
 # DRAM bytes (read + write) of one k_transform_data_backward launch per image,
-# from an ncu capture of 16 images (35.43 MB); traffic grows with the images
+# from an ncu capture of 16 images (35.42 MB); traffic grows with the images
 # processed
-BWD_DRAM_BYTES_PER_IMAGE = 35.43e6 / 16
+BWD_DRAM_BYTES_PER_IMAGE = 35.42e6 / 16
 
 
 def parse():
