@@ -1,11 +1,10 @@
-"""A warp's lanes without a point (sets whose size is not a multiple of 32, the
-end of an image) walk a trajectory from the domain's centre with a zero cotangent.
-Where that trajectory overflows and those of the call's own points do not, nothing
-of it may reach dtheta: 0 * inf is NaN.
+"""A warp's lanes without a point (sets whose size is not a multiple of 32, the end of
+an image) bring nothing into dtheta, whatever the field does away from the call's own
+points: a trajectory that overflows would, with a zero cotangent too (0 * inf is NaN).
 
 The points lie in cells whose field is zero and all others expand by e^80 a step
-(A = 4000 at 50 steps; the midpoint map by 3281), so that the centre's trajectory
-is infinite after a few steps.  The basis is the identity: dtheta is dL/dA.  It is
+(A = 4000 at 50 steps; the midpoint map by 3281): a trajectory from the domain's
+centre, say, is infinite after a few steps.  The basis is the identity: dtheta is dL/dA.  It is
 compared with the same points in full blocks of 256, filled up with more points of
 the zero cells whose cotangent is zero: the same sums in another order (1e-5).
 """
